@@ -56,7 +56,7 @@ struct SocsGeom {
   int KX;          // rows of the x twiddle table, max(NFM, NBM)
 };
 
-// Largest number of kernel slices the spectral stage splits a (clip, set) into.
+// Largest number of kernel slices the adjoint's spectral stage splits a (clip, set) into.
 constexpr int kSocsMaxSplit = 8;
 
 // Fill geometry; returns KL_OK or KL_ERR_UNSUPPORTED with a message.  With
@@ -66,10 +66,9 @@ int socs_geometry(int Lx, int Ly, int Nx, int Ny, SocsGeom* g, bool adjoint = fa
 
 // Device workspace sizes.
 size_t socs_partial_bytes(const SocsGeom& g, int nclips);
-size_t socs_spectrum_bytes(const SocsGeom& g, int nclips, int nsets, int nsplit);
 size_t socs_table_x_elems(const SocsGeom& g);  // float2 elements of tx
 size_t socs_table_y_elems(const SocsGeom& g);  // float2 elements of ty
-// kernel slices per (clip, set) for a launch of `nclips` clips
+// kernel slices per (clip, set) of the adjoint's spectral launch of `nclips` clips
 int socs_choose_split(const SocsGeom& g, int nclips, int nsets, int K);
 
 // Plan-time twiddle tables (stream-ordered).
@@ -78,12 +77,9 @@ int socs_build_tables(const SocsGeom& g, float2* tx, float2* ty, cudaStream_t st
 // Launchers (stream-ordered).  Buffers are device pointers.
 int socs_launch_forward(const SocsGeom& g, const float2* tx, const float2* ty, const float* masks,
                         int nclips, float2* partial, cudaStream_t st);
-int socs_launch_spectral(const SocsGeom& g, const float2* partial, int nclips, const float2* H,
-                         const float* lam, int K, int nsets, int nsplit, float2* T,
-                         cudaStream_t st);
 // spc: strips per CTA of the inverse kernel (0 = chosen from the batch size)
 int socs_launch_inverse(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T,
-                        int nclips, int nsets, int nsplit, float* images, cudaStream_t st, int spc = 0);
+                        int nclips, int nsets, float* images, cudaStream_t st, int spc = 0);
 // Image synthesis on the tensor cores (socs_synth_tc.cu): the inverse stage as
 // an FP16x3 split GEMM of the row coefficients against a cos/sin basis.
 bool synth_tc_supported(const SocsGeom& g);
@@ -92,7 +88,7 @@ bool synth_tc_aligned(const float* images);  // TMA stores need 16-byte aligned 
 // basis [Lx][Kp] as FP16 hi and lo halves (each Lx * Kp * 2 bytes)
 int synth_tc_build_basis(const SocsGeom& g, void* bhi, void* blo, cudaStream_t st);
 // err: device status word, set to a nonzero code if a pipeline wait times out
-int synth_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int nsplit, const void* bhi,
+int synth_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, const void* bhi,
                     const void* blo, int nimg, float* images, int* err, cudaStream_t st);
 // The mask transform (strip partial band spectra) on the tensor cores
 // (socs_fwd_tc.cu), in place of socs_launch_forward; thi / tlo: the transposed
@@ -108,7 +104,7 @@ bool vjp_tc_supported(const SocsGeom& g);
 // transposed row-DFT basis [64][Lx] as FP16 hi and lo halves (each 64 * Lx * 2 bytes)
 int vjp_tc_build_basis_t(const SocsGeom& g, void* thi, void* tlo, cudaStream_t st);
 // bhi / blo: the synthesis basis of synth_tc_build_basis (Kp = 64)
-int vjp_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int nclips, int nsets, int nsplit,
+int vjp_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int nclips, int nsets,
                   const void* bhi, const void* blo, const void* thi, const void* tlo, const float* targets,
                   float alpha, float thr, float* images, double* loss, float2* gpart, int* err, cudaStream_t st);
 // centred band of FT_r2c (DC at the band centre), complex64 nby x nbx per clip
@@ -120,7 +116,7 @@ int socs_launch_band(const SocsGeom& g, const float2* partial, int nclips, float
 // period Lx x Ly, bands up to 4N+1 <= 256.  Five stream-ordered stages:
 //   row_fwd  mask rows -> row bins R[y][fx], fx in [0, Nx]       (HBM-bound)
 //   col_fwd  R -> band spectrum, |fy| <= Ny                      (small)
-//   spectral band -> intensity spectrum T (cluster of G/32 CTAs per image)
+//   spectral band -> intensity spectrum T (spectral.cu)
 //   col_inv  T -> per-row coefficients Q[y][b], b in [0, 2Nx]    (small)
 //   row_inv  Q rows -> image rows                                (HBM-bound)
 // ---------------------------------------------------------------------------
@@ -145,12 +141,10 @@ __host__ __device__ inline bool gen_t2_in_smem(const GenGeom& g) { return (size_
 int gen_geometry(int Lx, int Ly, int Nx, int Ny, GenGeom* g);
 size_t gen_rowbins_bytes(const GenGeom& g, int nrows_img, int nbins);  // R / Q buffers
 size_t gen_band_bytes(const GenGeom& g, int n, int nparts, int nrows, int ncols);
-size_t gen_T_bytes(const GenGeom& g, int nimg, int nsplit);
 size_t gen_table_elems(const GenGeom& g);  // twb + twl + tw2 + rootLy (float2)
 int gen_build_tables(const GenGeom& g, float2* tables, cudaStream_t st);
-// kernel slices per image of a spectral launch with `per_sm` resident CTAs per SM
-// (2 for the forward core, 1 for the adjoint's)
-int gen_choose_split(const GenGeom& g, int nimg, int K, int per_sm = 2);
+// kernel slices per image of the adjoint's spectral launch
+int gen_choose_split(const GenGeom& g, int nimg, int K);
 int gen_choose_parts(const GenGeom& g, int n, int ncols);
 
 // stage launchers (device pointers, stream-ordered)
@@ -158,9 +152,7 @@ int gen_launch_rowfwd(const GenGeom& g, const float2* tables, const float* src, 
                       cudaStream_t st);
 int gen_launch_colfwd(const GenGeom& g, const float2* tables, const float2* R, int n, int ncols, int Yb,
                       float scale, int nparts, float2* band, cudaStream_t st);
-int gen_launch_spectral(const GenGeom& g, const float2* band, int nparts, int nclips, const float2* H,
-                        const float* lam, int K, int nsets, int nsplit, float2* T, cudaStream_t st);
-int gen_launch_colinv(const GenGeom& g, const float2* tables, const float2* T, int nimg, int nsplit, int A,
+int gen_launch_colinv(const GenGeom& g, const float2* tables, const float2* T, int nimg, int A,
                       int nbins, float2* Q, cudaStream_t st);
 int gen_launch_rowinv(const GenGeom& g, const float2* tables, const float2* Q, int nimg, int nbins,
                       float* images, cudaStream_t st);
@@ -177,6 +169,35 @@ int gen_launch_gradT(const GenGeom& g, const float2* gam, int nclips, int nparts
 int gen_launch_vjp_source(const GenGeom& g, const float2* band, int nparts, const float2* gband, int gparts,
                           int nimg, int nsets, const float2* Hs, int S, const float* Jw, const int* src_id,
                           int nsplit, float* grad_src, cudaStream_t st);
+
+// ---------------------------------------------------------------------------
+// Spectral core (spectral.cu), shared by both pipelines: band spectra ->
+// sum_k lambda_k |E_k|^2 -> its spectrum T.
+// ---------------------------------------------------------------------------
+struct SpecGeom {
+  int Nx, Ny, nbx, nby, nf, ntx, nty;  // as in SocsGeom
+  int G;                               // spectral grid, the smallest multiple of 32 >= 4N+1
+  int Lx, Ly, dx, dy;                  // period and one-pixel shift of odd periods
+  int ta, tb;                          // strides of T(a, b)
+};
+SpecGeom spec_geometry(const SocsGeom& g);
+SpecGeom spec_geometry(const GenGeom& g);
+// Largest number of kernel slices of one image.
+constexpr int kSpecMaxSplit = 64;
+int spec_choose_split(const SpecGeom& g, int nimg, int K);
+// float2 elements of the `part` buffer of a launch (what its CTAs hold of an image)
+size_t spec_part_elems(const SpecGeom& g, int nimg, int nsplit);
+// the kernels in the core's layout: float2 elements of one, and the conversion of
+// nk of them from the kernel layout
+size_t spec_kernel_elems(const SpecGeom& g);
+int spec_columns(const SpecGeom& g, const float2* H, int nk, float2* HT, cudaStream_t st);
+// band: nparts partial band spectra [nby][nf] per clip, summed and times scale.
+// H: kernels of all sets in the core's layout, or (natural) the kernel layout.  T
+// receives one spectrum per image.
+// done: nimg counters, zero before the first launch and left zero by each.
+int spec_launch(const SpecGeom& g, const float2* band, int nparts, float scale, int nimg, const float2* H, bool natural,
+                const float* lam, int K, int nsets, int nsplit, float2* part, float2* T,
+                unsigned* done, cudaStream_t st);
 
 }  // namespace kl
 

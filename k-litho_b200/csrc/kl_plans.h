@@ -13,10 +13,15 @@ struct kl_socs_plan_s {
   int K = 0, nsets = 0, max_clips = 0;
   int device = 0;
   bool adjoint = false;
-  float2* H = nullptr;       // nsets x K x nby x nbx
+  void* buffers = nullptr;   // the allocation that the device pointers below lie in
+  float2* H = nullptr;       // nsets x K x nby x nbx (adjoint plans)
+  float2* HT = nullptr;      // the same in the spectral core's layout
+  unsigned* done = nullptr;  // slice counters of the spectral core
+  kl::SpecGeom sg{};
   float* lam = nullptr;      // nsets x K
   float2* partial = nullptr; // max_clips strip partials
-  float2* T = nullptr;       // intensity spectra (clip x set x kernel slice)
+  float2* T = nullptr;       // intensity spectra
+  float2* part = nullptr;    // the spectral core's partial sums
   float2* tx = nullptr;      // plan-time twiddle tables
   float2* ty = nullptr;
   float* stage_in = nullptr; // host-entry staging (lazily allocated)
@@ -34,7 +39,7 @@ struct kl_socs_plan_s {
   bool timing = false;
   std::vector<cudaEvent_t> events;
   // launch shape chosen by kl_socs_autotune for batches of tune_clips clips
-  int tcap = 0;  // clip x kernel-slice products the spectra buffer holds
+  size_t part_cap = 0;  // float2 elements of `part`
   int tune_clips = 0, tune_nsplit = 0, tune_spc = 0;  // tune_spc < 0: tensor-core synthesis
   // synthesis engine of the specialised pipeline (KL_SYNTH_*), the tensor-core
   // basis (FP16 hi / lo halves, [Lx][Kp]) and its pipeline status word
@@ -92,7 +97,7 @@ namespace kl {
 int vjp_supported(const SocsGeom& g);
 size_t vjp_gpart_bytes(const SocsGeom& g, int nimg);
 int vjp_launch_inverse(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T,
-                       int nclips, int nsets, int nsplit, const float* targets, float alpha,
+                       int nclips, int nsets, const float* targets, float alpha,
                        float thr, float* images, double* loss, float2* gpart, cudaStream_t st);
 int vjp_launch_spectral(const SocsGeom& g, const float2* partial, const float2* gpart, int nclips,
                         const float2* H, const float* lam, int K, int nsets, int nsplit,

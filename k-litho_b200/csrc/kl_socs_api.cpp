@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "kl_internal.h"
+#include "kl_early.h"
 #include "kl_plans.h"
 
 namespace {
@@ -27,29 +28,22 @@ void free_plan(kl_socs_plan p) {
     }
     if (p->hev[i]) cudaEventDestroy(p->hev[i]);
   }
-  cudaFree(p->H);
-  cudaFree(p->lam);
-  cudaFree(p->partial);
-  cudaFree(p->T);
-  cudaFree(p->tx);
-  cudaFree(p->ty);
+  cudaFree(p->buffers);
   cudaFree(p->stage_in);
   cudaFree(p->stage_out);
-  cudaFree(p->gpart);
-  cudaFree(p->gam);
-  cudaFree(p->Tg);
-  cudaFree(p->gtab);
-  cudaFree(p->R);
-  cudaFree(p->band);
-  cudaFree(p->Q);
-  cudaFree(p->gband);
-  cudaFree(p->bhi);
-  cudaFree(p->blo);
-  cudaFree(p->status);
-  cudaFree(p->thi);
-  cudaFree(p->tlo);
   delete p;
 }
+
+// A plan's device buffers are pieces of one allocation: every cudaMalloc costs
+// 0.1 ms and more, and a plan made inside a call (kl_hopkins_image) pays for it.
+struct Pieces {
+  std::vector<std::pair<void**, size_t>> list;
+  template <typename T>
+  void add(T** p, size_t bytes) {
+    list.emplace_back(reinterpret_cast<void**>(p), (std::max<size_t>(bytes, 16) + 255) & ~size_t(255));
+  }
+  int allocate(void** base) const;
+};
 
 int alloc(void** ptr, size_t bytes, const char* what) {
   cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 16);
@@ -57,6 +51,18 @@ int alloc(void** ptr, size_t bytes, const char* what) {
     kl::set_error(std::string("cudaMalloc(") + what + "): " + cudaGetErrorString(e));
     cudaGetLastError();
     return KL_ERR_NOMEM;
+  }
+  return KL_OK;
+}
+
+int Pieces::allocate(void** base) const {
+  size_t total = 0;
+  for (const auto& e : list) total += e.second;
+  if (int rc = alloc(base, total, "plan buffers")) return rc;
+  char* c = static_cast<char*>(*base);
+  for (const auto& e : list) {
+    *e.first = c;
+    c += e.second;
   }
   return KL_OK;
 }
@@ -88,7 +94,7 @@ void launch_shape(kl_socs_plan p, int nclips, int* nsplit, int* spc) {
     *nsplit = p->tune_nsplit;
     *spc = p->tune_spc;
   } else {
-    *nsplit = kl::socs_choose_split(p->g, nclips, p->nsets, p->K);
+    *nsplit = kl::spec_choose_split(p->sg, nclips * p->nsets, p->K);
     *spc = 0;
   }
 }
@@ -99,8 +105,8 @@ int run_forward_gen(kl_socs_plan p, const float* masks, int nclips, float* image
                     const cudaEvent_t* ev4) {
   const kl::GenGeom& g = p->gg;
   const int nimg = nclips * p->nsets;
-  int nsplit = kl::gen_choose_split(g, nimg, p->K);
-  if (p->tune_clips == nclips && p->tune_nsplit > 0) nsplit = p->tune_nsplit;
+  int nsplit, spc;
+  launch_shape(p, nclips, &nsplit, &spc);
   const int nparts = kl::gen_choose_parts(g, nclips, g.nf);
   int rc;
   if ((rc = stage_mark(p, st, ev4, 0))) return rc;
@@ -109,10 +115,11 @@ int run_forward_gen(kl_socs_plan p, const float* masks, int nclips, float* image
                                   p->band, st)))
     return rc;
   if ((rc = stage_mark(p, st, ev4, 1))) return rc;
-  if ((rc = kl::gen_launch_spectral(g, p->band, nparts, nclips, p->H, p->lam, p->K, p->nsets, nsplit, p->T, st)))
+  if ((rc = kl::spec_launch(p->sg, p->band, nparts, 1.0f, nimg, p->HT, false, p->lam, p->K, p->nsets, nsplit, p->part,
+                            p->T, p->done, st)))
     return rc;
   if ((rc = stage_mark(p, st, ev4, 2))) return rc;
-  if ((rc = kl::gen_launch_colinv(g, p->gtab, p->T, nimg, nsplit, 2 * g.Ny, g.ntx, p->Q, st))) return rc;
+  if ((rc = kl::gen_launch_colinv(g, p->gtab, p->T, nimg, 2 * g.Ny, g.ntx, p->Q, st))) return rc;
   if ((rc = kl::gen_launch_rowinv(g, p->gtab, p->Q, nimg, g.ntx, images, st))) return rc;
   return stage_mark(p, st, ev4, 3);
 }
@@ -135,8 +142,48 @@ bool use_tc_forward(kl_socs_plan p, int nclips, const float* masks) {
   return p->tune_clips == nclips && p->tune_nsplit > 0 && p->tune_spc == -2;
 }
 
+// the spectral core of the specialised pipeline, from the strip partials
+int spectral(kl_socs_plan p, int nclips, int nsplit, cudaStream_t st) {
+  return kl::spec_launch(p->sg, p->partial, p->g.nS, 1.0f / ((float)p->g.Lx * (float)p->g.Ly), nclips * p->nsets, p->HT,
+                         false, p->lam, p->K, p->nsets, nsplit, p->part, p->T, p->done, st);
+}
+
+// buffers of the spectral core: the kernels in its layout (and, for the adjoint,
+// the kernel layout), spectra for any batch up to max_clips, slice counters
+void spectral_pieces(kl_socs_plan p, Pieces& mem) {
+  const kl::SpecGeom& g = p->sg;
+  const size_t nk = (size_t)p->K * p->nsets, nimg = (size_t)p->max_clips * p->nsets;
+  for (int n = 1; n <= p->max_clips; ++n)
+    p->part_cap = std::max(p->part_cap, kl::spec_part_elems(g, n * p->nsets,
+                                                            kl::spec_choose_split(g, n * p->nsets, p->K)));
+  mem.add(&p->HT, sizeof(float2) * nk * kl::spec_kernel_elems(g));
+  if (p->adjoint) mem.add(&p->H, sizeof(float2) * nk * g.nby * g.nbx);
+  mem.add(&p->lam, sizeof(float) * nk);
+  mem.add(&p->T, sizeof(float2) * nimg * g.nty * g.ntx);
+  mem.add(&p->part, sizeof(float2) * p->part_cap);
+  mem.add(&p->done, sizeof(unsigned) * nimg);
+}
+
+// a new plan's kernels are zero, as are its counters; the default stream's work
+// is done on return
+int finish_plan(kl_socs_plan p) {
+  const kl::SpecGeom& g = p->sg;
+  const size_t nk = (size_t)p->K * p->nsets;
+  cudaMemsetAsync(p->HT, 0, sizeof(float2) * nk * kl::spec_kernel_elems(g), nullptr);
+  if (p->H) cudaMemsetAsync(p->H, 0, sizeof(float2) * nk * g.nby * g.nbx, nullptr);
+  cudaMemsetAsync(p->lam, 0, sizeof(float) * nk, nullptr);
+  cudaMemsetAsync(p->done, 0, sizeof(unsigned) * p->max_clips * p->nsets, nullptr);
+  if (p->status) cudaMemsetAsync(p->status, 0, sizeof(int), nullptr);
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    kl::set_error(std::string("kl_socs_plan_create: ") + cudaGetErrorString(cudaGetLastError()));
+    return KL_ERR_CUDA;
+  }
+  return KL_OK;
+}
+
 int run_forward(kl_socs_plan p, const float* masks, int nclips, float* images, cudaStream_t st,
                 const cudaEvent_t* ev4 = nullptr) {
+  const kl::EarlyLaunch early(!ev4 && !p->timing);
   if (p->gen) return run_forward_gen(p, masks, nclips, images, st, ev4);
   int rc;
   if ((rc = stage_mark(p, st, ev4, 0))) return rc;
@@ -150,12 +197,11 @@ int run_forward(kl_socs_plan p, const float* masks, int nclips, float* images, c
     rc = kl::socs_launch_forward(p->g, p->tx, p->ty, masks, nclips, p->partial, st);
   if (rc) return rc;
   if ((rc = stage_mark(p, st, ev4, 1))) return rc;
-  rc = kl::socs_launch_spectral(p->g, p->partial, nclips, p->H, p->lam, p->K, p->nsets, nsplit,
-                                p->T, st);
+  rc = spectral(p, nclips, nsplit, st);
   if (rc) return rc;
   if ((rc = stage_mark(p, st, ev4, 2))) return rc;
-  rc = tc ? kl::synth_tc_launch(p->g, p->T, p->ty, nsplit, p->bhi, p->blo, nclips * p->nsets, images, p->status, st)
-          : kl::socs_launch_inverse(p->g, p->tx, p->ty, p->T, nclips, p->nsets, nsplit, images, st, spc);
+  rc = tc ? kl::synth_tc_launch(p->g, p->T, p->ty, p->bhi, p->blo, nclips * p->nsets, images, p->status, st)
+          : kl::socs_launch_inverse(p->g, p->tx, p->ty, p->T, nclips, p->nsets, images, st, spc);
   if (rc) return rc;
   return stage_mark(p, st, ev4, 3);
 }
@@ -191,48 +237,31 @@ int create_gen_plan(kl_socs_plan* plan, int Lx, int Ly, int Nx, int Ny, int nk, 
   p->nsets = nsets;
   p->max_clips = max_clips;
   cudaGetDevice(&p->device);
-  const size_t nb2 = (size_t)gg.nby * gg.nbx;
-  // spectra buffer: the largest (image, kernel slice) count any batch size or
-  // autotuned split needs
-  int tcap = 0, pmax = 0;
-  for (int n = 1; n <= max_clips; ++n) {
-    tcap = std::max(tcap, n * nsets * kl::gen_choose_split(gg, n * nsets, nk));
-    if (adjoint) tcap = std::max(tcap, n * nsets * kl::gen_choose_split(gg, n * nsets, nk, 1));
-    pmax = std::max(pmax, kl::gen_choose_parts(gg, n, gg.nf));
-  }
-  for (int ns = 1; ns <= kl::kGenMaxSplit; ns *= 2) tcap = std::max(tcap, std::min(ns, nk) * nsets);
-  p->tcap = tcap;
+  p->sg = kl::spec_geometry(gg);
+  int pmax = 0;
+  for (int n = 1; n <= max_clips; ++n) pmax = std::max(pmax, kl::gen_choose_parts(gg, n, gg.nf));
   p->nparts_max = pmax;
-  if ((rc = alloc((void**)&p->H, sizeof(float2) * nb2 * nk * nsets, "kernels")) ||
-      (rc = alloc((void**)&p->lam, sizeof(float) * (size_t)nk * nsets, "eigenvalues")) ||
-      (rc = alloc((void**)&p->gtab, sizeof(float2) * kl::gen_table_elems(gg), "tables")) ||
-      (rc = alloc((void**)&p->R, kl::gen_rowbins_bytes(gg, max_clips, gg.nf), "row bins")) ||
-      (rc = alloc((void**)&p->band, kl::gen_band_bytes(gg, max_clips, pmax, gg.nby, gg.nf), "band partials")) ||
-      (rc = alloc((void**)&p->T, kl::gen_T_bytes(gg, tcap, 1), "spectra")) ||
-      (rc = alloc((void**)&p->Q, kl::gen_rowbins_bytes(gg, max_clips * nsets, gg.ntx), "row coefficients")) ||
-      (rc = kl::gen_build_tables(gg, p->gtab, nullptr))) {
+  Pieces mem;
+  spectral_pieces(p, mem);
+  mem.add(&p->gtab, sizeof(float2) * kl::gen_table_elems(gg));
+  mem.add(&p->R, kl::gen_rowbins_bytes(gg, max_clips, gg.nf));
+  mem.add(&p->band, kl::gen_band_bytes(gg, max_clips, pmax, gg.nby, gg.nf));
+  mem.add(&p->Q, kl::gen_rowbins_bytes(gg, max_clips * nsets, gg.ntx));
+  if (adjoint) {
+    int gmax = 0, slices = 0;
+    for (int n = 1; n <= max_clips; ++n) {
+      gmax = std::max(gmax, kl::gen_choose_parts(gg, n * nsets, gg.ntx));
+      slices = std::max(slices, n * nsets * kl::gen_choose_split(gg, n * nsets, nk));
+    }
+    p->gparts_max = gmax;
+    mem.add(&p->gband, kl::gen_band_bytes(gg, max_clips * nsets, gmax, gg.nty, gg.ntx));
+    mem.add(&p->gam, sizeof(float2) * gg.nby * gg.nbx * slices);
+    mem.add(&p->Tg, sizeof(float2) * (size_t)max_clips * gg.nf * gg.nby);
+  }
+  if ((rc = mem.allocate(&p->buffers)) || (rc = kl::gen_build_tables(gg, p->gtab, nullptr)) || (rc = finish_plan(p))) {
     free_plan(p);
     return rc;
   }
-  if (adjoint) {
-    int gmax = 0;
-    for (int n = 1; n <= max_clips; ++n) gmax = std::max(gmax, kl::gen_choose_parts(gg, n * nsets, gg.ntx));
-    p->gparts_max = gmax;
-    if ((rc = alloc((void**)&p->gband, kl::gen_band_bytes(gg, max_clips * nsets, gmax, gg.nty, gg.ntx),
-                    "dL/dI bands")) ||
-        (rc = alloc((void**)&p->gam, sizeof(float2) * nb2 * tcap, "adjoint partials")) ||
-        (rc = alloc((void**)&p->Tg, sizeof(float2) * (size_t)max_clips * gg.nf * gg.nby, "gradient spectra"))) {
-      free_plan(p);
-      return rc;
-    }
-  }
-  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
-    kl::set_error(std::string("kl_socs_plan_create: ") + cudaGetErrorString(cudaGetLastError()));
-    free_plan(p);
-    return KL_ERR_CUDA;
-  }
-  cudaMemset(p->H, 0, sizeof(float2) * nb2 * nk * nsets);
-  cudaMemset(p->lam, 0, sizeof(float) * (size_t)nk * nsets);
   *plan = p;
   return KL_OK;
 }
@@ -259,64 +288,39 @@ int create_plan(kl_socs_plan* plan, int Lx, int Ly, int Nx, int Ny, int nk, int 
   p->nsets = nsets;
   p->max_clips = max_clips;
   cudaGetDevice(&p->device);
-  const size_t nb2 = (size_t)g.nby * g.nbx;
-  if ((rc = alloc((void**)&p->H, sizeof(float2) * nb2 * nk * nsets, "kernels")) ||
-      (rc = alloc((void**)&p->lam, sizeof(float) * (size_t)nk * nsets, "eigenvalues")) ||
-      (rc = alloc((void**)&p->partial, kl::socs_partial_bytes(g, max_clips), "partials")) ||
-      (rc = alloc((void**)&p->tx, sizeof(float2) * kl::socs_table_x_elems(g), "x twiddles")) ||
-      (rc = alloc((void**)&p->ty, sizeof(float2) * kl::socs_table_y_elems(g), "y twiddles"))) {
-    free_plan(p);
-    return rc;
-  }
-  // spectra buffer: the largest clips x slices product any batch size needs
-  int tcap = 0;
-  for (int n = 1; n <= max_clips; ++n) {
-    const int c = n * kl::socs_choose_split(g, n, nsets, nk);
-    tcap = c > tcap ? c : tcap;
-  }
-  p->tcap = tcap;
-  if ((rc = alloc((void**)&p->T, kl::socs_spectrum_bytes(g, tcap, nsets, 1), "spectra")) ||
-      (rc = kl::socs_build_tables(g, p->tx, p->ty, nullptr))) {
-    free_plan(p);
-    return rc;
-  }
+  p->sg = kl::spec_geometry(g);
+  Pieces mem;
+  spectral_pieces(p, mem);
+  mem.add(&p->partial, kl::socs_partial_bytes(g, max_clips));
+  mem.add(&p->tx, sizeof(float2) * kl::socs_table_x_elems(g));
+  mem.add(&p->ty, sizeof(float2) * kl::socs_table_y_elems(g));
   if (kl::synth_tc_supported(g)) {
     const size_t bb = (size_t)g.Lx * kl::synth_tc_kp(g) * 2;
-    if ((rc = alloc(&p->bhi, bb, "synthesis basis")) || (rc = alloc(&p->blo, bb, "synthesis basis")) ||
-        (rc = alloc((void**)&p->status, sizeof(int), "status word")) ||
-        (rc = kl::synth_tc_build_basis(g, p->bhi, p->blo, nullptr))) {
-      free_plan(p);
-      return rc;
-    }
-    cudaMemset(p->status, 0, sizeof(int));
+    mem.add(&p->bhi, bb);
+    mem.add(&p->blo, bb);
+    mem.add(&p->status, sizeof(int));
     // the transposed basis of the row DFTs: the tensor-core mask transform and,
     // on adjoint plans, the row DFT of dL/dI
     p->vjp_tc = adjoint && kl::synth_tc_kp(g) == 64 && kl::vjp_tc_supported(g);
     if (kl::fwd_tc_supported(g) || p->vjp_tc) {
       const size_t tb = (size_t)64 * g.Lx * 2;
-      if ((rc = alloc(&p->thi, tb, "row DFT basis")) || (rc = alloc(&p->tlo, tb, "row DFT basis")) ||
-          (rc = kl::vjp_tc_build_basis_t(g, p->thi, p->tlo, nullptr))) {
-        free_plan(p);
-        return rc;
-      }
+      mem.add(&p->thi, tb);
+      mem.add(&p->tlo, tb);
     }
   }
   if (adjoint) {
-    const size_t nb2s = (size_t)g.nby * g.nbx;
-    if ((rc = alloc((void**)&p->gpart, kl::vjp_gpart_bytes(g, max_clips * nsets), "dL/dI partials")) ||
-        (rc = alloc((void**)&p->gam, sizeof(float2) * nb2s * tcap * nsets, "adjoint partials")) ||
-        (rc = alloc((void**)&p->Tg, sizeof(float2) * (size_t)max_clips * g.nty * g.ntx, "gradient spectra"))) {
-      free_plan(p);
-      return rc;
-    }
+    int slices = 0;  // the largest clips x slices product any batch size needs
+    for (int n = 1; n <= max_clips; ++n) slices = std::max(slices, n * kl::socs_choose_split(g, n, nsets, nk));
+    mem.add(&p->gpart, kl::vjp_gpart_bytes(g, max_clips * nsets));
+    mem.add(&p->gam, sizeof(float2) * g.nby * g.nbx * slices * nsets);
+    mem.add(&p->Tg, sizeof(float2) * (size_t)max_clips * g.nty * g.ntx);
   }
-  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
-    kl::set_error(std::string("kl_socs_plan_create: ") + cudaGetErrorString(cudaGetLastError()));
+  if ((rc = mem.allocate(&p->buffers)) || (rc = kl::socs_build_tables(g, p->tx, p->ty, nullptr)) ||
+      (p->bhi && (rc = kl::synth_tc_build_basis(g, p->bhi, p->blo, nullptr))) ||
+      (p->thi && (rc = kl::vjp_tc_build_basis_t(g, p->thi, p->tlo, nullptr))) || (rc = finish_plan(p))) {
     free_plan(p);
-    return KL_ERR_CUDA;
+    return rc;
   }
-  cudaMemset(p->H, 0, sizeof(float2) * nb2 * nk * nsets);
-  cudaMemset(p->lam, 0, sizeof(float) * (size_t)nk * nsets);
   *plan = p;
   return KL_OK;
 }
@@ -329,8 +333,8 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
             float* images, float* grad, double* loss, cudaStream_t st) {
   const kl::GenGeom& g = p->gg;
   const int nimg = nclips * p->nsets;
-  const int ns = kl::gen_choose_split(g, nimg, p->K);
-  const int ns_adj = kl::gen_choose_split(g, nimg, p->K, 1);
+  const int ns = kl::spec_choose_split(p->sg, nimg, p->K);
+  const int ns_adj = kl::gen_choose_split(g, nimg, p->K);
   const int nparts = kl::gen_choose_parts(g, nclips, g.nf);
   const int gparts = kl::gen_choose_parts(g, nimg, g.ntx);
   int rc;
@@ -338,9 +342,10 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
   if ((rc = kl::gen_launch_colfwd(g, p->gtab, p->R, nclips, g.nf, g.Ny, 1.0f / ((float)g.Lx * (float)g.Ly), nparts,
                                   p->band, st)))
     return rc;
-  if ((rc = kl::gen_launch_spectral(g, p->band, nparts, nclips, p->H, p->lam, p->K, p->nsets, ns, p->T, st)))
+  if ((rc = kl::spec_launch(p->sg, p->band, nparts, 1.0f, nimg, p->HT, false, p->lam, p->K, p->nsets, ns, p->part, p->T,
+                            p->done, st)))
     return rc;
-  if ((rc = kl::gen_launch_colinv(g, p->gtab, p->T, nimg, ns, 2 * g.Ny, g.ntx, p->Q, st))) return rc;
+  if ((rc = kl::gen_launch_colinv(g, p->gtab, p->T, nimg, 2 * g.Ny, g.ntx, p->Q, st))) return rc;
   KL_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(double) * (size_t)nimg, st));
   if ((rc = kl::gen_launch_rowvjp(g, p->gtab, p->Q, nimg, p->nsets, targets, alpha, threshold, images, loss, st)))
     return rc;
@@ -349,11 +354,24 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
                                         ns_adj, p->gam, st)))
     return rc;
   if ((rc = kl::gen_launch_gradT(g, p->gam, nclips, p->nsets * ns_adj, p->Tg, st))) return rc;
-  if ((rc = kl::gen_launch_colinv(g, p->gtab, p->Tg, nclips, 1, g.Ny, g.nf, p->Q, st))) return rc;
+  if ((rc = kl::gen_launch_colinv(g, p->gtab, p->Tg, nclips, g.Ny, g.nf, p->Q, st))) return rc;
   if ((rc = kl::gen_launch_rowinv(g, p->gtab, p->Q, nclips, g.nf, grad, st))) return rc;
   p->last_vjp_clips = nclips;
   p->last_nparts = nparts;
   p->last_gparts = gparts;
+  return KL_OK;
+}
+}  // namespace
+
+namespace {
+// host kernels -> H (device, kernel layout) -> the spectral core's layout, and the
+// eigenvalues; done on return
+int upload_kernels(kl_socs_plan p, int set, const float2* h, float2* H, const float* scales) {
+  const size_t nb2 = (size_t)p->g.nby * p->g.nbx, k0 = (size_t)set * p->K;
+  KL_CUDA_TRY(cudaMemcpy(H, h, sizeof(float2) * nb2 * p->K, cudaMemcpyHostToDevice));
+  if (int rc = kl::spec_columns(p->sg, H, p->K, p->HT + k0 * kl::spec_kernel_elems(p->sg), nullptr)) return rc;
+  KL_CUDA_TRY(cudaMemcpy(p->lam + k0, scales, sizeof(float) * p->K, cudaMemcpyHostToDevice));
+  KL_CUDA_TRY(cudaStreamSynchronize(nullptr));
   return KL_OK;
 }
 }  // namespace
@@ -395,22 +413,20 @@ int kl_socs_vjp(kl_socs_plan p, const float* masks, const float* targets, int nc
   if (p->gen) return vjp_gen(p, masks, targets, nclips, alpha, threshold, images, grad, loss, st);
   const kl::SocsGeom& g = p->g;
   int rc;
-  const int ns1 = kl::socs_choose_split(g, nclips, p->nsets, p->K);
   if (p->synth == KL_SYNTH_TENSOR_CORES && use_tc_forward(p, nclips, masks))
     rc = kl::fwd_tc_launch(g, masks, nclips, p->ty, p->thi, p->tlo, p->partial, p->status, st);
   else
     rc = kl::socs_launch_forward(g, p->tx, p->ty, masks, nclips, p->partial, st);
   if (rc) return rc;
-  if ((rc = kl::socs_launch_spectral(g, p->partial, nclips, p->H, p->lam, p->K, p->nsets, ns1, p->T, st)))
-    return rc;
+  if ((rc = spectral(p, nclips, kl::spec_choose_split(p->sg, nclips * p->nsets, p->K), st))) return rc;
   KL_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(double) * (size_t)nclips * p->nsets, st));
   // image, resist, loss and the row DFT of dL/dI: on the tensor cores where
   // the plan has them, unless it asks for the CUDA-core engine
   const bool tca = p->vjp_tc && p->synth != KL_SYNTH_CUDA_CORES &&
                    (((uintptr_t)targets | (uintptr_t)images) & 15) == 0;
-  rc = tca ? kl::vjp_tc_launch(g, p->T, p->ty, nclips, p->nsets, ns1, p->bhi, p->blo, p->thi, p->tlo, targets, alpha,
+  rc = tca ? kl::vjp_tc_launch(g, p->T, p->ty, nclips, p->nsets, p->bhi, p->blo, p->thi, p->tlo, targets, alpha,
                                threshold, images, loss, p->gpart, p->status, st)
-           : kl::vjp_launch_inverse(g, p->tx, p->ty, p->T, nclips, p->nsets, ns1, targets, alpha, threshold, images,
+           : kl::vjp_launch_inverse(g, p->tx, p->ty, p->T, nclips, p->nsets, targets, alpha, threshold, images,
                                     loss, p->gpart, st);
   if (rc) return rc;
   const int ns2 = kl::socs_choose_split(g, nclips, p->nsets, p->K);
@@ -421,8 +437,8 @@ int kl_socs_vjp(kl_socs_plan p, const float* masks, const float* targets, int nc
   // the gradient is a band-limited synthesis like the image: on the tensor
   // cores unless the plan asks for the CUDA-core engine
   const bool tcg = p->bhi && p->synth != KL_SYNTH_CUDA_CORES && kl::synth_tc_aligned(grad);
-  rc = tcg ? kl::synth_tc_launch(g, p->Tg, p->ty, 1, p->bhi, p->blo, nclips, grad, p->status, st)
-           : kl::socs_launch_inverse(g, p->tx, p->ty, p->Tg, nclips, 1, 1, grad, st);
+  rc = tcg ? kl::synth_tc_launch(g, p->Tg, p->ty, p->bhi, p->blo, nclips, grad, p->status, st)
+           : kl::socs_launch_inverse(g, p->tx, p->ty, p->Tg, nclips, 1, grad, st);
   if (rc) return rc;
   p->last_vjp_clips = nclips;
   return KL_OK;
@@ -471,22 +487,29 @@ int kl_socs_set_kernels(kl_socs_plan p, int set, const float* re, const float* i
   const size_t nb2 = (size_t)p->g.nby * p->g.nbx;
   std::vector<float2> h(nb2 * p->K);
   for (size_t i = 0; i < h.size(); ++i) h[i] = make_float2(re[i], im[i]);
-  KL_CUDA_TRY(cudaMemcpy(p->H + (size_t)set * p->K * nb2, h.data(), sizeof(float2) * h.size(),
-                         cudaMemcpyHostToDevice));
-  KL_CUDA_TRY(cudaMemcpy(p->lam + (size_t)set * p->K, scales, sizeof(float) * p->K,
-                         cudaMemcpyHostToDevice));
-  return KL_OK;
+  // in the kernel layout: kept by adjoint plans, else only on the way to the
+  // spectral core's layout
+  float2* H = p->H ? p->H + (size_t)set * p->K * nb2 : nullptr;
+  void* tmp = nullptr;
+  int rc;
+  if (!H) {
+    if ((rc = kl::scratch_alloc(&tmp, sizeof(float2) * h.size(), nullptr, "kernels"))) return rc;
+    H = static_cast<float2*>(tmp);
+  }
+  rc = upload_kernels(p, set, h.data(), H, scales);
+  if (tmp) kl::scratch_free(tmp, nullptr);
+  return rc;
 }
 
 int kl_socs_set_kernels_device(kl_socs_plan p, int set, const float2* H_dev, const float* lam_dev,
                                cudaStream_t st) {
   KL_CHECK_ARG(p && H_dev && lam_dev, "kl_socs_set_kernels_device: NULL argument");
   KL_CHECK_ARG(set >= 0 && set < p->nsets, "kl_socs_set_kernels_device: set out of range");
-  const size_t nb2 = (size_t)p->g.nby * p->g.nbx;
-  KL_CUDA_TRY(cudaMemcpyAsync(p->H + (size_t)set * p->K * nb2, H_dev, sizeof(float2) * nb2 * p->K,
-                              cudaMemcpyDeviceToDevice, st));
-  KL_CUDA_TRY(cudaMemcpyAsync(p->lam + (size_t)set * p->K, lam_dev, sizeof(float) * p->K,
-                              cudaMemcpyDeviceToDevice, st));
+  const size_t nb2 = (size_t)p->g.nby * p->g.nbx, k0 = (size_t)set * p->K;
+  if (p->H)
+    KL_CUDA_TRY(cudaMemcpyAsync(p->H + k0 * nb2, H_dev, sizeof(float2) * nb2 * p->K, cudaMemcpyDeviceToDevice, st));
+  if (int rc = kl::spec_columns(p->sg, H_dev, p->K, p->HT + k0 * kl::spec_kernel_elems(p->sg), st)) return rc;
+  KL_CUDA_TRY(cudaMemcpyAsync(p->lam + k0, lam_dev, sizeof(float) * p->K, cudaMemcpyDeviceToDevice, st));
   return KL_OK;
 }
 

@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "kl_early.h"
 #include "kl_internal.h"
 #include "kl_plans.h"
 
@@ -48,6 +49,9 @@ void destroy_batch(kl_socs_batch_s* b) {
 
 // fork on `origin`, one branch per plan, join back on `origin`
 int enqueue_branches(kl_socs_batch_s* b, const float* const* masks, const int* nclips, float* const* images) {
+  // kernels that wait on the SMs for their predecessor's end would keep the other
+  // branches' kernels off them (0.59 against 0.57 ms for 96 clips of three sizes)
+  const kl::EarlyLaunch in_order(false);
   KL_CUDA_TRY(cudaEventRecord(b->fork, b->origin));
   for (size_t i = 0; i < b->plans.size(); ++i) {
     KL_CUDA_TRY(cudaStreamWaitEvent(b->branch[i], b->fork, 0));
@@ -81,11 +85,8 @@ int kl_socs_autotune(kl_socs_plan p, const float* masks, int nclips, float* imag
   const bool timing = p->timing;
   p->timing = false;
   std::vector<int> splits, spcs;
-  // the spectra buffer holds tcap (clip, slice) pairs per kernel set on the
-  // specialised kernels, tcap (image, slice) pairs on the general pipeline
-  const int per_slice = p->gen ? nclips * p->nsets : nclips;
-  for (int ns = 1; ns <= kl::kSocsMaxSplit; ns *= 2)
-    if (ns * per_slice <= p->tcap && ns <= p->K) splits.push_back(ns);
+  for (int ns : {1, 2, 4, 8})
+    if (ns <= p->K && kl::spec_part_elems(p->sg, nclips * p->nsets, ns) <= p->part_cap) splits.push_back(ns);
   // strips per CTA of the synthesis: specialised kernels only
   if (!p->gen)
     for (int c = 1; c <= 16 && c <= p->g.nS; c *= 2) spcs.push_back(c);

@@ -15,26 +15,21 @@
 //     bins.  The strip's J rows then go through a J-point warp FFT along y
 //     (rows are J-periodic in the strip), giving the strip's partial band
 //     spectrum D_s[fy][fx], |fy| <= Ny.
-//  2. k_socs_spectral (on-chip; CTAs per clip, kernel set and kernel slice)
-//     Sums the strip partials into the band spectrum, then for each kernel
-//     of its slice forms H_k . M, runs a pruned 2-D inverse FFT on a G x G
-//     grid (G >= 4N+1, so |E_k|^2 is sampled without aliasing) with warp FFTs
-//     in shared memory and accumulates lambda_k |E_k|^2 in registers.  A
-//     forward 2-D FFT of that intensity gives the slice's share of the exact
+//  2. k_spectral (spectral.cu; on-chip, CTAs per clip, kernel set and kernel
+//     slice)
+//     Sums the strip partials into the band spectrum and forms the exact
 //     band-limited intensity spectrum T[a][b], |a| <= 2Ny, 0 <= b <= 2Nx.
 //  3. k_socs_inverse  (HBM-bound; writes the image once)
-//     One CTA per (image, strip).  Sums the slices of T, forms the strip's
-//     rows by a J-point warp FFT along y, and each warp synthesises a row of
+//     One CTA per (image, strip).  Forms the strip's rows by a J-point warp FFT along y, and each warp synthesises a row of
 //     Lx real pixels from its 2Nx+1 bins with a real-output length-P inverse
 //     DFT per lane.
 //
 // Twiddle factors that depend on the clip size are made once per plan
 // (k_socs_tables, exact double-precision arguments) and read from L2.
 // Only the strip partials, T and the tables pass through global memory.
-#include <climits>
-
 #include "kl_device.cuh"
 #include "kl_internal.h"
+#include "kl_launch.cuh"
 
 namespace kl {
 
@@ -120,9 +115,6 @@ int socs_geometry(int Lx, int Ly, int Nx, int Ny, SocsGeom* g, bool adjoint) {
 size_t socs_partial_bytes(const SocsGeom& g, int nclips) {
   return sizeof(float2) * (size_t)nclips * g.nS * g.nby * g.nf;
 }
-size_t socs_spectrum_bytes(const SocsGeom& g, int nclips, int nsets, int nsplit) {
-  return sizeof(float2) * (size_t)nclips * nsets * nsplit * g.nty * g.ntx;
-}
 size_t socs_table_x_elems(const SocsGeom& g) { return (size_t)g.KX * g.V; }
 size_t socs_table_y_elems(const SocsGeom& g) { return (size_t)g.nS * g.nty; }
 
@@ -180,6 +172,8 @@ __global__ void __launch_bounds__(kThreads) k_socs_forward(const float* __restri
   const float* mask = masks + (size_t)clip * g.Lx * g.Ly;
 
   for (int i = threadIdx.x; i < NFM * V; i += kThreads) twf[i] = __ldg(tx + i);
+  dep_wait();
+  dep_launch();
   __syncthreads();
 
   for (int jj = warp; jj < J; jj += kWarps) {
@@ -233,9 +227,6 @@ __global__ void __launch_bounds__(kThreads) k_socs_forward(const float* __restri
   }
 }
 
-// ---------------------------------------------------------------------------
-// 2. spectral core: band spectrum -> sum_k lambda_k |E_k|^2 -> its spectrum T
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ void load_band(const float2* __restrict__ partial, const SocsGeom& g,
                                           int clip, float2* Cm) {
   const float inv = 1.0f / ((float)g.Lx * (float)g.Ly);
@@ -251,153 +242,6 @@ __device__ __forceinline__ void load_band(const float2* __restrict__ partial, co
   }
 }
 
-template <int RG>
-__global__ void __launch_bounds__(kThreads) k_socs_spectral(const float2* __restrict__ partial,
-                                                            const SocsGeom g,
-                                                            const float2* __restrict__ H,
-                                                            const float* __restrict__ lam, int K,
-                                                            float2* __restrict__ Tout) {
-  constexpr int G = 32 * RG;
-  constexpr int GP = G + 1;  // padded row pitch (bank-conflict free columns)
-  constexpr int CW = G / kWarps;  // columns owned by each warp
-  extern __shared__ float4 smem4[];
-  float2* Cm = reinterpret_cast<float2*>(smem4);  // [nby][nbx] band spectrum / (Lx Ly)
-  float2* E1 = Cm + g.nby * g.nbx;                // [nby][GP] stage-1 rows; later T1 [G][ntx]
-  const int e1n = g.nby * GP > G * g.ntx ? g.nby * GP : G * g.ntx;
-  float* Is = reinterpret_cast<float*>(E1 + e1n);  // [G][GP] intensity
-  float2* Zs = reinterpret_cast<float2*>(Is + G * GP);  // [warps][G]
-
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int clip = blockIdx.x, set = blockIdx.y, split = blockIdx.z;
-  const int nsets = gridDim.y, nsplit = gridDim.z;
-  const int k0 = (int)(((long long)K * split) / nsplit), k1 = (int)(((long long)K * (split + 1)) / nsplit);
-  const int br = (int)(__brev((unsigned)lane) >> 27);
-
-  load_band(partial, g, clip, Cm);
-  __syncthreads();
-
-  WarpFFT<RG, +1> wi;
-  wi.init(lane);
-  float acc[CW][RG];
-#pragma unroll
-  for (int t = 0; t < CW; ++t)
-#pragma unroll
-    for (int q = 0; q < RG; ++q) acc[t][q] = 0.f;
-
-  const size_t nb2 = (size_t)g.nby * g.nbx;
-  const float2* Hs = H + (size_t)set * K * nb2;
-  for (int k = k0; k < k1; ++k) {
-    const float2* Hk = Hs + (size_t)k * nb2;
-    const float lk = __ldg(lam + set * K + k);
-    // stage 1: rows fy, inverse FFT along x of H_k . M (two rows per pass)
-    for (int r0 = warp; r0 < g.nby; r0 += 2 * kWarps) {
-      float2 va[RG], vb[RG];
-      const int r1 = r0 + kWarps;
-      const bool has1 = r1 < g.nby;
-#pragma unroll
-      for (int j = 0; j < RG; ++j) {
-        const int n = lane + 32 * j;
-        const int fx = n <= g.Nx ? n : (n >= G - g.Nx ? n - G : INT_MIN);
-        va[j] = make_float2(0.f, 0.f);
-        vb[j] = make_float2(0.f, 0.f);
-        if (fx != INT_MIN) {
-          const int o0 = r0 * g.nbx + fx + g.Nx;
-          va[j] = cmul(__ldg(Hk + o0), Cm[o0]);
-          if (has1) {
-            const int o1 = r1 * g.nbx + fx + g.Nx;
-            vb[j] = cmul(__ldg(Hk + o1), Cm[o1]);
-          }
-        }
-      }
-      wi.run(va, lane);
-      wi.run(vb, lane);
-#pragma unroll
-      for (int q1 = 0; q1 < RG; ++q1) {
-        E1[r0 * GP + q1 + RG * br] = va[q1];
-        if (has1) E1[r1 * GP + q1 + RG * br] = vb[q1];
-      }
-    }
-    __syncthreads();
-    // stage 2: columns q, inverse FFT along y; accumulate lambda |E|^2
-#pragma unroll
-    for (int t = 0; t < CW; ++t) {
-      const int q = warp + kWarps * t;
-      float2 vv[RG];
-#pragma unroll
-      for (int j = 0; j < RG; ++j) {
-        const int n = lane + 32 * j;
-        const int fy = n <= g.Ny ? n : (n >= G - g.Ny ? n - G : INT_MIN);
-        vv[j] = (fy != INT_MIN) ? E1[(fy + g.Ny) * GP + q] : make_float2(0.f, 0.f);
-      }
-      wi.run(vv, lane);
-#pragma unroll
-      for (int q1 = 0; q1 < RG; ++q1) acc[t][q1] = fmaf(lk, cabs2(vv[q1]), acc[t][q1]);
-    }
-    __syncthreads();
-  }
-
-  // intensity to shared memory: I[p][q], p = q1 + RG*brev(lane), q = warp + 8t
-#pragma unroll
-  for (int t = 0; t < CW; ++t)
-#pragma unroll
-    for (int q1 = 0; q1 < RG; ++q1) Is[(q1 + RG * br) * GP + warp + kWarps * t] = acc[t][q1];
-  __syncthreads();
-
-  // stage A: forward FFT along x of row pairs packed as one complex row
-  WarpFFT<RG, -1> wfw;
-  wfw.init(lane);
-  float2* T1 = E1;  // [G][ntx]
-  float2* Zw = Zs + warp * G;
-  for (int pp = warp; pp < G / 2; pp += kWarps) {
-    const int p1 = 2 * pp, p2 = 2 * pp + 1;
-    float2 vv[RG];
-#pragma unroll
-    for (int j = 0; j < RG; ++j) {
-      const int q = lane + 32 * j;
-      vv[j] = make_float2(Is[p1 * GP + q], Is[p2 * GP + q]);
-    }
-    wfw.run(vv, lane);
-#pragma unroll
-    for (int q1 = 0; q1 < RG; ++q1) Zw[q1 + RG * br] = vv[q1];
-    __syncwarp();
-    for (int b = lane; b < g.ntx; b += 32) {
-      const float2 za = Zw[b];
-      const float2 zb = cconj(Zw[(G - b) & (G - 1)]);
-      const float2 x1 = cscale(cadd(za, zb), 0.5f);
-      const float2 d = cscale(csub(za, zb), 0.5f);  // x2 = d / i
-      T1[p1 * g.ntx + b] = x1;
-      T1[p2 * g.ntx + b] = make_float2(d.y, -d.x);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-
-  // stage B: forward FFT along y of each kept column b; scale and shift phase
-  const float invg = 1.0f / ((float)G * (float)G);
-  float2* To = Tout + (((size_t)clip * nsets + set) * nsplit + split) * g.nty * g.ntx;
-  for (int b = warp; b < g.ntx; b += kWarps) {
-    float2 vv[RG];
-#pragma unroll
-    for (int j = 0; j < RG; ++j) vv[j] = T1[(lane + 32 * j) * g.ntx + b];
-    wfw.run(vv, lane);
-#pragma unroll
-    for (int q1 = 0; q1 < RG; ++q1) {
-      const int bin = q1 + RG * br;
-      const int a = bin <= G / 2 ? bin : bin - G;
-      if (a >= -2 * g.Ny && a <= 2 * g.Ny) {
-        float2 v = cscale(vv[q1], invg);
-        if (g.dx | g.dy) {
-          // odd periods: the reference's shifts move the image by one pixel
-          const float2 ph1 = expi2pi_frac(-(long long)a * g.dy, g.Ly);
-          const float2 ph2 = expi2pi_frac(-(long long)b * g.dx, g.Lx);
-          v = cmul(v, cmul(ph1, ph2));
-        }
-        To[(a + 2 * g.Ny) * g.ntx + b] = v;
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // 3. inverse: intensity spectrum -> image rows
 // ---------------------------------------------------------------------------
@@ -406,7 +250,7 @@ __global__ void __launch_bounds__(kThreads) k_socs_inverse(const float2* __restr
                                                            const SocsGeom g,
                                                            const float2* __restrict__ tx,
                                                            const float2* __restrict__ ty,
-                                                           int nsplit, int spc,
+                                                           int spc,
                                                            float* __restrict__ images) {
   constexpr int J = 32 * RJ;
   constexpr int QP = NBM + 1;
@@ -419,19 +263,17 @@ __global__ void __launch_bounds__(kThreads) k_socs_inverse(const float2* __restr
   const int img = blockIdx.y;
   const int s0 = blockIdx.x * spc, s1 = min(g.nS, s0 + spc);  // this CTA's strips
   const size_t tsz = (size_t)g.nty * g.ntx;
-  const float2* Ti = T + (size_t)img * nsplit * tsz;
+  const float2* Ti = T + (size_t)img * tsz;
 
-  // once per CTA: the image's band spectrum (slices summed), the x twiddles,
-  // and the zero columns b >= ntx of the row coefficients
-#pragma unroll 4
-  for (int i = threadIdx.x; i < (int)tsz; i += kThreads) {
-    float2 v = __ldg(Ti + i);
-    for (int p = 1; p < nsplit; ++p) v = cadd(v, __ldg(Ti + p * tsz + i));
-    Ts[i] = v;
-  }
+  // once per CTA: the x twiddles, the zero columns b >= ntx of the row
+  // coefficients and the image's band spectrum
 #pragma unroll 4
   for (int i = threadIdx.x; i < NBM * V; i += kThreads) twi[i] = __ldg(tx + i);
   for (int i = threadIdx.x; i < J * QP; i += kThreads) Qs[i] = make_float2(0.f, 0.f);
+  dep_wait();
+  dep_launch();
+#pragma unroll 4
+  for (int i = threadIdx.x; i < (int)tsz; i += kThreads) Ts[i] = __ldg(Ti + i);
   float2 ph_next = make_float2(0.f, 0.f);
   if (threadIdx.x < g.nty) ph_next = __ldg(ty + (size_t)s0 * g.nty + threadIdx.x);
   __syncthreads();
@@ -531,6 +373,7 @@ __global__ void k_socs_band(const float2* __restrict__ partial, const SocsGeom g
   extern __shared__ float4 smem4[];
   float2* Cm = reinterpret_cast<float2*>(smem4);
   const int clip = blockIdx.x;
+  dep_wait();
   load_band(partial, g, clip, Cm);
   __syncthreads();
   const int yh = (g.Ly + 1) / 2, xh = (g.Lx + 1) / 2;
@@ -575,13 +418,13 @@ int launch_fwd(const SocsGeom& g, const float2* tx, const float2* ty, const floa
   auto kern = k_socs_forward<P, V, NFM, RJ>;
   int rc = set_smem(kern, sm);
   if (rc) return rc;
-  kern<<<dim3(g.nS, nclips), kThreads, sm, st>>>(masks, g, tx, ty, partial);
-  return check_launch("k_socs_forward");
+  KL_CUDA_TRY(launch_dependent(kern, dim3(g.nS, nclips), kThreads, sm, st, masks, g, tx, ty, partial));
+  return KL_OK;
 }
 
 template <int P, int V, int NBM, int RJ>
 int launch_inv(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T, int nimg,
-               int nsplit, float* images, cudaStream_t st, int spc) {
+               float* images, cudaStream_t st, int spc) {
   size_t sm = sizeof(float2) * ((size_t)NBM * V + (size_t)32 * RJ * (NBM + 1) +
                                 (size_t)g.nty * g.ntx + g.nty);
   auto kern = k_socs_inverse<P, V, NBM, RJ>;
@@ -594,23 +437,10 @@ int launch_inv(const SocsGeom& g, const float2* tx, const float2* ty, const floa
     while (spc < 8 && spc * 2 <= g.nS && (long long)nimg * ((g.nS + 2 * spc - 1) / (2 * spc)) >= 4 * 148) spc *= 2;
   }
   spc = spc < g.nS ? spc : g.nS;
-  kern<<<dim3((g.nS + spc - 1) / spc, nimg), kThreads, sm, st>>>(T, g, tx, ty, nsplit, spc, images);
-  return check_launch("k_socs_inverse");
+  KL_CUDA_TRY(launch_dependent(kern, dim3((g.nS + spc - 1) / spc, nimg), kThreads, sm, st, T, g, tx, ty, spc, images));
+  return KL_OK;
 }
 
-template <int RG>
-int launch_spec(const SocsGeom& g, const float2* partial, int nclips, const float2* H,
-                const float* lam, int K, int nsets, int nsplit, float2* T, cudaStream_t st) {
-  constexpr int G = 32 * RG, GP = G + 1;
-  size_t e1n = (size_t)g.nby * GP > (size_t)G * g.ntx ? (size_t)g.nby * GP : (size_t)G * g.ntx;
-  size_t sm = sizeof(float2) * ((size_t)g.nby * g.nbx + e1n) + sizeof(float) * (size_t)G * GP +
-              sizeof(float2) * (size_t)kWarps * G;
-  auto kern = k_socs_spectral<RG>;
-  int rc = set_smem(kern, sm);
-  if (rc) return rc;
-  kern<<<dim3(nclips, nsets, nsplit), kThreads, sm, st>>>(partial, g, H, lam, K, T);
-  return check_launch("k_socs_spectral");
-}
 }  // namespace
 
 #define KL_PV_LIST(X, A, B) \
@@ -632,26 +462,13 @@ int socs_launch_forward(const SocsGeom& g, const float2* tx, const float2* ty, c
   return KL_ERR_UNSUPPORTED;
 }
 
-int socs_launch_spectral(const SocsGeom& g, const float2* partial, int nclips, const float2* H,
-                         const float* lam, int K, int nsets, int nsplit, float2* T,
-                         cudaStream_t st) {
-  if (nclips <= 0) return KL_OK;
-  switch (g.G) {
-    case 32: return launch_spec<1>(g, partial, nclips, H, lam, K, nsets, nsplit, T, st);
-    case 64: return launch_spec<2>(g, partial, nclips, H, lam, K, nsets, nsplit, T, st);
-    case 128: return launch_spec<4>(g, partial, nclips, H, lam, K, nsets, nsplit, T, st);
-  }
-  set_error("socs_launch_spectral: unsupported spectral grid");
-  return KL_ERR_UNSUPPORTED;
-}
-
 int socs_launch_inverse(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T,
-                        int nclips, int nsets, int nsplit, float* images, cudaStream_t st, int spc) {
+                        int nclips, int nsets, float* images, cudaStream_t st, int spc) {
   if (nclips <= 0) return KL_OK;
   const int RJ = g.J / 32, nimg = nclips * nsets;
 #define KL_INV(P_, V_, N_, R_)                               \
   if (g.P == P_ && g.V == V_ && g.NBM == N_ && RJ == R_) \
-    return launch_inv<P_, V_, N_, R_>(g, tx, ty, T, nimg, nsplit, images, st, spc);
+    return launch_inv<P_, V_, N_, R_>(g, tx, ty, T, nimg, images, st, spc);
   KL_PV_LIST(KL_INV, 32, 1)
   KL_PV_LIST(KL_INV, 32, 2)
   KL_PV_LIST(KL_INV, 64, 1)

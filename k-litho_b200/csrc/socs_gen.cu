@@ -17,14 +17,8 @@
 //  col_fwd   the row bins' DFT along y, kept for |fy| <= Ny: 32-point warp FFTs
 //            over strips of 32 rows spaced Ly/32 apart when 32 divides Ly,
 //            otherwise a direct sum; strips are split over `nparts` partial bands.
-//  spectral  per (image, kernel slice) a cluster of RG = G/32 CTAs; CTA c holds
-//            the grid columns x = c + RG j (j < 32): the band rows are folded
-//            mod 32 with the twiddle e^{2 pi i fx c/G} and inverse transformed by
-//            a 32-point warp FFT, the columns by G-point warp FFTs; the K fields'
-//            lambda |E|^2 stay in registers.  The intensity is transformed back
-//            (y by the transposed warp FFT straight from registers, x by a
-//            32-point FFT) and the RG CTAs sum their contributions to the
-//            intensity spectrum T through distributed shared memory.
+//  spectral  (spectral.cu) the band's K fields, their lambda |E|^2 and its
+//            spectrum T, on chip.
 //  col_inv   T's columns synthesised along y for every image row (strip FFTs
 //            or a direct sum), giving the rows' coefficients Q[y][b], b <= 2Nx.
 //  row_inv   (HBM-bound) each warp synthesises image rows from Q: lane l'
@@ -41,6 +35,7 @@
 
 #include "kl_device.cuh"
 #include "kl_internal.h"
+#include "kl_launch.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -125,15 +120,12 @@ size_t gen_band_bytes(const GenGeom& g, int n, int nparts, int nrows, int ncols)
   (void)g;
   return sizeof(float2) * (size_t)n * nparts * nrows * ncols;
 }
-size_t gen_T_bytes(const GenGeom& g, int nimg, int nsplit) {
-  return sizeof(float2) * (size_t)nimg * nsplit * g.ntx * g.nty;
-}
 size_t gen_table_elems(const GenGeom& g) { return off_rly(g) + (size_t)g.Ly; }
 
-int gen_choose_split(const GenGeom& g, int nimg, int K, int per_sm) {
+int gen_choose_split(const GenGeom& g, int nimg, int K) {
   // kernel slices per image: the count whose CTAs fill the GPU's resident
   // slots most evenly (waves x work per CTA), with slices of at least 3 kernels
-  const long long slots = (long long)kSMs * per_sm, ctas = (long long)g.RG * nimg;
+  const long long slots = kSMs, ctas = (long long)g.RG * nimg;
   int best = 1;
   double best_t = 1e30;
   for (int ns = 1; ns <= kGenMaxSplit && (ns == 1 || K / ns >= 3); ns *= 2) {
@@ -223,6 +215,8 @@ __global__ void __launch_bounds__(kT) k_gen_rowfwd(const float* __restrict__ src
   const float2* twl = tables + off_twl(g);
   const float2* tw2 = tables + off_tw2(g);
   for (int i = threadIdx.x; i < 32 * g.NBX; i += kT) tl[i] = __ldg(twl + i);
+  dep_wait();
+  dep_launch();
   __syncthreads();
   const int V = g.Vf, nch = (V + 31) / 32, nt = (nbins + 31) / 32;
   for (int row = blockIdx.x * kW + warp; row < nrows; row += gridDim.x * kW) {
@@ -287,6 +281,8 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int fx = blockIdx.x * kW + warp;
   const int n = blockIdx.y, part = blockIdx.z, nparts = gridDim.z;
+  dep_wait();
+  dep_launch();
   if (fx >= ncols) return;  // whole warp; no block-wide barrier below
   const int nyo = 2 * Yb + 1, Ly = g.Ly;
   const float2* Rn = R + (size_t)n * Ly * ncols;
@@ -357,191 +353,9 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R,
 }
 
 // ---------------------------------------------------------------------------
-// 3. spectral core: band -> sum_k lambda_k |E_k|^2 -> T[img][split][b][a]
+// 3. col_inv: T[img][b][a + A] -> Q[img][y][b] = w_b sum_a T e^{2 pi i a y/Ly}
 // ---------------------------------------------------------------------------
-// Shared memory (float2 units): the band half Mh [nby][nf] and stage-1 rows
-// E1 [nby][33] during the kernel loop; afterwards, over the same space, the
-// per-warp FFT rows Zw [8][G] and the y-transformed intensity Ys [nty][33];
-// then the G roots of unity.
-__host__ __device__ inline size_t gen_spec_smem_elems(const GenGeom& g) {
-  const size_t r0 = (size_t)g.nby * g.nf + (size_t)g.nby * 33;
-  const size_t r1 = (size_t)kW * g.G + (size_t)g.nty * 33;
-  return (r0 > r1 ? r0 : r1) + g.G;
-}
-
-template <int RG>
-__global__ void __launch_bounds__(kT, 2) k_gen_spectral(const float2* __restrict__ band, int nparts,
-                                                        const GenGeom g, const float2* __restrict__ H,
-                                                        const float* __restrict__ lam, int K, int nsets,
-                                                        float2* __restrict__ Tout) {
-  constexpr int G = 32 * RG;
-  constexpr int CW = 32 / kW;  // columns per warp
-  cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ float4 smem4[];
-  float2* base = reinterpret_cast<float2*>(smem4);
-  float2* Mh = base;                    // [nby][nf]
-  float2* E1 = Mh + g.nby * g.nf;       // [nby][33]
-  float2* Zw = base;                    // [kW][G]   (after the kernel loop)
-  float2* Ys = Zw + kW * G;             // [nty][33] (after the kernel loop)
-  const size_t r0 = (size_t)g.nby * g.nf + (size_t)g.nby * 33;
-  const size_t r1 = (size_t)kW * G + (size_t)g.nty * 33;
-  float2* rootG = base + (r0 > r1 ? r0 : r1);  // [G] e^{+2 pi i m / G}
-
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c = blockIdx.x;  // grid column class = rank in the cluster
-  const int img = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z;
-  const int clip = img / nsets, set = img - clip * nsets;
-  const int k0 = (int)(((long long)K * split) / nsplit), k1 = (int)(((long long)K * (split + 1)) / nsplit);
-  const int br = brev5(lane);
-  const int nf = g.nf, nby = g.nby, nbx = g.nbx, Nx = g.Nx, Ny = g.Ny;
-
-  for (int i = threadIdx.x; i < G; i += kT) rootG[i] = expi2pi_frac(i, G);
-  __syncthreads();
-  // band half, parts summed, times e^{2 pi i fx c / G} (keeps the conjugate
-  // symmetry M'[fy][-fx] = conj M'[-fy][fx])
-  {
-    const size_t per = (size_t)nby * nf;
-    const float2* b0 = band + (size_t)clip * nparts * per;
-    for (int i = threadIdx.x; i < nby * nf; i += kT) {
-      const int fx = i % nf;
-      float2 v = __ldg(b0 + i);
-      for (int p = 1; p < nparts; ++p) v = cadd(v, __ldg(b0 + p * per + i));
-      Mh[i] = cmul(v, rootG[(fx * c) & (G - 1)]);
-    }
-  }
-  __syncthreads();
-
-  WarpFFT<1, +1> w1;
-  w1.init(lane);
-  WarpFFT<RG, +1> wi;
-  wi.init(lane);
-  float acc[CW][RG];
-#pragma unroll
-  for (int t = 0; t < CW; ++t)
-#pragma unroll
-    for (int q = 0; q < RG; ++q) acc[t][q] = 0.f;
-
-  const size_t nb2 = (size_t)nby * nbx;
-  const float2* Hs = H + (size_t)set * K * nb2;
-  const int fxs = lane - 32 * ((lane + Nx) / 32);  // smallest fx >= -Nx with fx = lane (mod 32)
-  // the kernel rows come from L2: each warp keeps the loads of its next row in
-  // flight while it folds and transforms the current one (the next kernel's
-  // first row after its last), so their latency overlaps the work
-  float2 hn[kGenMaxFold];
-  if (k0 < k1 && warp < nby) gen_load_hrow(Hs + (size_t)k0 * nb2, warp, nbx, Nx, fxs, hn);
-  for (int k = k0; k < k1; ++k) {
-    const float2* Hk = Hs + (size_t)k * nb2;
-    const float lk = __ldg(lam + set * K + k);
-    // stage 1: band rows folded mod 32, then a 32-point inverse FFT over the lanes
-    for (int r = warp; r < nby; r += kW) {
-      float2 h[kGenMaxFold];
-#pragma unroll
-      for (int t = 0; t < kGenMaxFold; ++t) h[t] = hn[t];
-      if (r + kW < nby) gen_load_hrow(Hk, r + kW, nbx, Nx, fxs, hn);
-      else if (k + 1 < k1) gen_load_hrow(Hk + nb2, warp, nbx, Nx, fxs, hn);
-      float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int t = 0; t < kGenMaxFold; ++t) {
-        const int fx = fxs + 32 * t;
-        if (fx <= Nx) {
-          const float2 m = fx >= 0 ? Mh[r * nf + fx] : cconj(Mh[(nby - 1 - r) * nf - fx]);
-          v = cfma(h[t], m, v);
-        }
-      }
-      float2 vv[1] = {v};
-      w1.run(vv, lane);
-      E1[r * 33 + br] = vv[0];
-    }
-    __syncthreads();
-    // stage 2: the CTA's 32 columns, G-point inverse FFT along y
-#pragma unroll
-    for (int t = 0; t < CW; ++t) {
-      const int j = warp + kW * t;
-      float2 vv[RG];
-#pragma unroll
-      for (int i = 0; i < RG; ++i) {
-        const int n = lane + 32 * i;
-        const int fy = n <= Ny ? n : (n >= G - Ny ? n - G : INT_MIN);
-        vv[i] = fy != INT_MIN ? E1[(fy + Ny) * 33 + j] : make_float2(0.f, 0.f);
-      }
-      wi.run(vv, lane);
-#pragma unroll
-      for (int q = 0; q < RG; ++q) acc[t][q] = fmaf(lk, cabs2(vv[q]), acc[t][q]);
-    }
-    __syncthreads();
-  }
-
-  // y transform of the intensity columns, two real columns per complex FFT,
-  // straight from the registers' bit-reversed layout
-  WarpFFT<RG, -1> wf;
-  wf.init(lane);
-  float2* zw = Zw + warp * G;
-  const int A = 2 * Ny;
-#pragma unroll
-  for (int pr = 0; pr < CW / 2; ++pr) {
-    const int j0 = warp + kW * (2 * pr), j1 = warp + kW * (2 * pr + 1);
-    float2 vv[RG];
-#pragma unroll
-    for (int q = 0; q < RG; ++q) vv[q] = make_float2(acc[2 * pr][q], acc[2 * pr + 1][q]);
-    wf.run_rev(vv, lane);
-#pragma unroll
-    for (int i = 0; i < RG; ++i) zw[lane + 32 * i] = vv[i];
-    __syncwarp();
-    for (int a = -A + lane; a <= A; a += 32) {
-      const float2 za = zw[a & (G - 1)], zb = cconj(zw[(-a) & (G - 1)]);
-      const float2 y0 = cscale(cadd(za, zb), 0.5f);
-      const float2 d = cscale(csub(za, zb), 0.5f);
-      Ys[(a + A) * 33 + j0] = y0;
-      Ys[(a + A) * 33 + j1] = make_float2(d.y, -d.x);
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-  // x transform over the CTA's 32 columns: F[a][m] = sum_j Ys[a][j] e^{-2 pi i m j/32}
-  {
-    WarpFFT<1, -1> wx;
-    wx.init(lane);
-    for (int r = warp; r < g.nty; r += kW) {
-      float2 vv[1] = {Ys[r * 33 + lane]};
-      wx.run(vv, lane);
-      __syncwarp();
-      Ys[r * 33 + br] = vv[0];
-    }
-  }
-  cl.sync();
-  // T[b][a] = (1/G^2) sum_c e^{-2 pi i b c / G} F_c[a][b mod 32]; this CTA
-  // writes rows a in [a0, a1)
-  {
-    const int per = (g.nty + RG - 1) / RG;
-    const int a0 = c * per, a1 = min(g.nty, a0 + per), na = a1 - a0;
-    const float invg = 1.0f / ((float)G * (float)G);
-    float2* To = Tout + ((size_t)img * nsplit + split) * g.ntx * g.nty;
-    const float2* peers[RG];
-#pragma unroll
-    for (int cc = 0; cc < RG; ++cc) peers[cc] = cl.map_shared_rank(Ys, cc);
-    for (int i = threadIdx.x; i < na * g.ntx; i += kT) {
-      const int b = i / na, r = a0 + (i - b * na);
-      const int m = b & 31;
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int cc = 0; cc < RG; ++cc) s = cfma(peers[cc][r * 33 + m], cconj(rootG[(b * cc) & (G - 1)]), s);
-      s = cscale(s, invg);
-      if (g.dx | g.dy) {
-        // odd periods: the reference's shifts move the image by one pixel
-        const float2 ph1 = expi2pi_frac(-(long long)(r - A) * g.dy, g.Ly);
-        const float2 ph2 = expi2pi_frac(-(long long)b * g.dx, g.Lx);
-        s = cmul(s, cmul(ph1, ph2));
-      }
-      To[(size_t)b * g.nty + r] = s;
-    }
-  }
-  cl.sync();  // peers' shared memory stays valid until every CTA has read it
-}
-
-// ---------------------------------------------------------------------------
-// 4. col_inv: T[img][split][b][a + A] -> Q[img][y][b] = w_b sum_a T e^{2 pi i a y/Ly}
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kT) k_gen_colinv(const float2* __restrict__ T, int nsplit, int A, int nbins,
+__global__ void __launch_bounds__(kT) k_gen_colinv(const float2* __restrict__ T, int A, int nbins,
                                                    const GenGeom g, const float2* __restrict__ rly,
                                                    float2* __restrict__ Q, int spc) {
   extern __shared__ float4 smem4[];
@@ -551,12 +365,14 @@ __global__ void __launch_bounds__(kT) k_gen_colinv(const float2* __restrict__ T,
   const int lda = 2 * A + 1, qp = nbins + 1, Ly = g.Ly;
   const int img = blockIdx.y;
   const size_t tsz = (size_t)nbins * lda;
-  const float2* Ti = T + (size_t)img * nsplit * tsz;
+  const float2* Ti = T + (size_t)img * tsz;
   float2* Qi = Q + (size_t)img * Ly * nbins;
   WarpFFT<1, +1> wf;
   wf.init(lane);
   const int br = brev5(lane);
   const int s0 = blockIdx.x * spc, s1 = min(g.nS, s0 + spc);
+  dep_wait();
+  dep_launch();
   for (int s = s0; s < s1; ++s) {
     int nr = 32;
     if (g.ystrip) {
@@ -610,7 +426,7 @@ __global__ void __launch_bounds__(kT) k_gen_colinv(const float2* __restrict__ T,
 }
 
 // ---------------------------------------------------------------------------
-// 5. row_inv: Q[row][b] (b < nbins) -> out[row][x] = Re sum_b Q[b] e^{2 pi i b x/Lx}
+// 4. row_inv: Q[row][b] (b < nbins) -> out[row][x] = Re sum_b Q[b] e^{2 pi i b x/Lx}
 // ---------------------------------------------------------------------------
 template <int P>
 __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* __restrict__ Q, int nbins, int nrows,
@@ -629,6 +445,8 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* __restrict__ Q,
   if (t2_shared)
     for (int i = threadIdx.x; i < nch * g.NBX; i += kT) t2s[i] = __ldg(tables + off_tw2(g) + i);
   __syncthreads();
+  dep_wait();
+  dep_launch();
   const int nbp = (nbins + P - 1) / P * P;
   // each lane holds the coefficients b = lane + 32 t of its warp's row; the
   // next row's are loaded while the current one is synthesised
@@ -679,17 +497,6 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* __restrict__ Q,
   }
 }
 
-// slice partials of T summed into slice 0 (one pass over L2-resident data), so
-// that the column synthesis reads one spectrum per image
-__global__ void k_gen_sumT(float2* __restrict__ T, size_t tsz, int nsplit) {
-  float2* Ti = T + (size_t)blockIdx.y * nsplit * tsz;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < tsz; i += (size_t)gridDim.x * blockDim.x) {
-    float2 v = Ti[i];
-    for (int p = 1; p < nsplit; ++p) v = cadd(v, Ti[p * tsz + i]);
-    Ti[i] = v;
-  }
-}
-
 // centred FT_r2c band: M(ky,kx) = D(ky,kx) e^{-2 pi i (ky yh/Ly + kx xh/Lx)}
 __global__ void k_gen_bandout(const float2* __restrict__ band, int nparts, const GenGeom g,
                               float2* __restrict__ out) {
@@ -726,8 +533,8 @@ int launch_rowfwd_t(const GenGeom& g, const float2* tables, const float* src, in
   auto kern = k_gen_rowfwd<PF>;
   int rc = set_smem(kern, sm);
   if (rc) return rc;
-  kern<<<row_grid(nrows, 8), kT, sm, st>>>(src, nrows, g, tables, nbins, R);
-  return check_launch("k_gen_rowfwd");
+  KL_CUDA_TRY(launch_dependent(kern, row_grid(nrows, 8), kT, sm, st, src, nrows, g, tables, nbins, R));
+  return KL_OK;
 }
 
 template <int P>
@@ -738,36 +545,10 @@ int launch_rowinv_t(const GenGeom& g, const float2* tables, const float2* Q, int
   auto kern = k_gen_rowinv<P>;
   int rc = set_smem(kern, sm);
   if (rc) return rc;
-  kern<<<row_grid(nrows, 8), kT, sm, st>>>(Q, nbins, nrows, g, tables, out);
-  return check_launch("k_gen_rowinv");
+  KL_CUDA_TRY(launch_dependent(kern, row_grid(nrows, 8), kT, sm, st, Q, nbins, nrows, g, tables, out));
+  return KL_OK;
 }
 
-template <int RG>
-int launch_spectral_t(const GenGeom& g, const float2* band, int nparts, int nclips, const float2* H,
-                      const float* lam, int K, int nsets, int nsplit, float2* T, cudaStream_t st) {
-  const size_t sm = sizeof(float2) * gen_spec_smem_elems(g);
-  auto kern = k_gen_spectral<RG>;
-  int rc = set_smem(kern, sm);
-  if (rc) return rc;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(RG, nclips * nsets, nsplit);
-  cfg.blockDim = dim3(kT);
-  cfg.dynamicSmemBytes = sm;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = RG;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, band, nparts, g, H, lam, K, nsets, T);
-  if (e != cudaSuccess) {
-    set_error(std::string("k_gen_spectral: ") + cudaGetErrorString(e));
-    return KL_ERR_CUDA;
-  }
-  return check_launch("k_gen_spectral");
-}
 }  // namespace
 
 int gen_launch_rowfwd(const GenGeom& g, const float2* tables, const float* src, int nrows, float2* R,
@@ -793,34 +574,13 @@ int gen_launch_colfwd(const GenGeom& g, const float2* tables, const float2* R, i
     return KL_ERR_UNSUPPORTED;
   }
   dim3 grid((ncols + kW - 1) / kW, n, nparts);
-  k_gen_colfwd<<<grid, kT, 0, st>>>(R, ncols, Yb, g, tables + off_rly(g), scale, band);
-  return check_launch("k_gen_colfwd");
+  KL_CUDA_TRY(launch_dependent(k_gen_colfwd, grid, kT, 0, st, R, ncols, Yb, g, tables + off_rly(g), scale, band));
+  return KL_OK;
 }
 
-int gen_launch_spectral(const GenGeom& g, const float2* band, int nparts, int nclips, const float2* H,
-                        const float* lam, int K, int nsets, int nsplit, float2* T, cudaStream_t st) {
-  if (nclips <= 0) return KL_OK;
-  switch (g.RG) {
-    case 1: return launch_spectral_t<1>(g, band, nparts, nclips, H, lam, K, nsets, nsplit, T, st);
-    case 2: return launch_spectral_t<2>(g, band, nparts, nclips, H, lam, K, nsets, nsplit, T, st);
-    case 4: return launch_spectral_t<4>(g, band, nparts, nclips, H, lam, K, nsets, nsplit, T, st);
-    case 8: return launch_spectral_t<8>(g, band, nparts, nclips, H, lam, K, nsets, nsplit, T, st);
-  }
-  set_error("gen_launch_spectral: unsupported spectral grid");
-  return KL_ERR_UNSUPPORTED;
-}
-
-int gen_launch_colinv(const GenGeom& g, const float2* tables, const float2* T, int nimg, int nsplit, int A,
+int gen_launch_colinv(const GenGeom& g, const float2* tables, const float2* T, int nimg, int A,
                       int nbins, float2* Q, cudaStream_t st) {
   if (nimg <= 0) return KL_OK;
-  if (nsplit > 1) {
-    // fold the slices into slice 0 first (T is the caller's spectra buffer)
-    const size_t tsz = (size_t)nbins * (2 * A + 1);
-    const int bx = (int)std::min<size_t>((tsz + 255) / 256, 64);
-    k_gen_sumT<<<dim3(bx, nimg), 256, 0, st>>>(const_cast<float2*>(T), tsz, nsplit);
-    int rc = check_launch("k_gen_sumT");
-    if (rc) return rc;
-  }
   // a few strips per CTA so the image's T is reused from L1, enough CTAs to fill the GPU
   int spc = 1;
   while (spc < 8 && (long long)nimg * ((g.nS + 2 * spc - 1) / (2 * spc)) >= 4 * kSMs) spc *= 2;
@@ -828,8 +588,8 @@ int gen_launch_colinv(const GenGeom& g, const float2* tables, const float2* T, i
   int rc = set_smem(k_gen_colinv, sm);
   if (rc) return rc;
   dim3 grid((g.nS + spc - 1) / spc, nimg);
-  k_gen_colinv<<<grid, kT, sm, st>>>(T, nsplit, A, nbins, g, tables + off_rly(g), Q, spc);  // reads slice 0
-  return check_launch("k_gen_colinv");
+  KL_CUDA_TRY(launch_dependent(k_gen_colinv, grid, kT, sm, st, T, A, nbins, g, tables + off_rly(g), Q, spc));
+  return KL_OK;
 }
 
 int gen_launch_rowinv(const GenGeom& g, const float2* tables, const float2* Q, int nimg, int nbins, float* images,

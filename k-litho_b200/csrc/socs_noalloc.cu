@@ -18,6 +18,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <mutex>
 #include <string>
 
@@ -96,12 +97,19 @@ extern "C" int kl_socs_forward_noalloc(const float* masks_dev, int nclips, int L
   kl::SocsGeom g;
   int rc = kl::socs_geometry(Lx, Ly, Nx, Ny, &g);
   if (rc) return rc;
-  const int nsplit = kl::socs_choose_split(g, nclips, 1, nk);
+  const kl::SpecGeom sg = kl::spec_geometry(g);
   const size_t b_tx = up256(sizeof(float2) * kl::socs_table_x_elems(g));
   const size_t b_ty = up256(sizeof(float2) * kl::socs_table_y_elems(g));
   const size_t b_part = up256(kl::socs_partial_bytes(g, nclips));
-  const size_t b_T = up256(kl::socs_spectrum_bytes(g, nclips, 1, nsplit));
+  const size_t b_T = up256(sizeof(float2) * (size_t)nclips * g.nty * g.ntx);
   const size_t need = b_tx + b_ty + b_part + b_T;
+  // what the spectral core's CTAs hold of an image, and its counters, pass through
+  // the image buffer: it is written only afterwards
+  const size_t b_cnt = up256(sizeof(unsigned) * nclips);
+  const size_t room = sizeof(float) * (size_t)Lx * Ly * nclips;
+  auto core_bytes = [&](int ns) { return 256 + b_cnt + sizeof(float2) * kl::spec_part_elems(sg, nclips, ns); };
+  int nsplit = kl::spec_choose_split(sg, nclips, nk);
+  while (nsplit > 1 && core_bytes(nsplit) > room) --nsplit;
   if (need > kNoallocScratchBytes) {
     kl::set_error("kl_socs_forward_noalloc: " + std::to_string(nclips) + " clips of " +
                   std::to_string(Lx) + "x" + std::to_string(Ly) + " need " + std::to_string(need) +
@@ -116,11 +124,15 @@ extern "C" int kl_socs_forward_noalloc(const float* masks_dev, int nclips, int L
   float2* ty = reinterpret_cast<float2*>(p + b_tx);
   float2* partial = reinterpret_cast<float2*>(p + b_tx + b_ty);
   float2* T = reinterpret_cast<float2*>(p + b_tx + b_ty + b_part);
+  unsigned* done = reinterpret_cast<unsigned*>((reinterpret_cast<uintptr_t>(images_dev) + 255) & ~uintptr_t(255));
+  float2* core = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(done) + b_cnt);
   cudaStream_t st = (cudaStream_t)stream;
   if ((rc = kl::socs_build_tables(g, tx, ty, st))) return rc;
   if ((rc = kl::socs_launch_forward(g, tx, ty, masks_dev, nclips, partial, st))) return rc;
-  if ((rc = kl::socs_launch_spectral(g, partial, nclips, reinterpret_cast<const float2*>(kernels_dev),
-                                     scales_dev, nk, 1, nsplit, T, st)))
+  KL_CUDA_TRY(cudaMemsetAsync(done, 0, sizeof(unsigned) * nclips, st));
+  if ((rc = kl::spec_launch(sg, partial, g.nS, 1.0f / ((float)Lx * (float)Ly), nclips,
+                            reinterpret_cast<const float2*>(kernels_dev), true, scales_dev, nk, 1, nsplit, core, T,
+                            done, st)))
     return rc;
-  return kl::socs_launch_inverse(g, tx, ty, T, nclips, 1, nsplit, images_dev, st);
+  return kl::socs_launch_inverse(g, tx, ty, T, nclips, 1, images_dev, st);
 }

@@ -43,6 +43,7 @@
 
 #include "kl_device.cuh"
 #include "kl_internal.h"
+#include "kl_launch.cuh"
 #include "kl_tc.cuh"
 
 namespace kl {
@@ -106,7 +107,7 @@ __global__ void k_synth_basis(int Lx, int ntx, int Kp, __half* __restrict__ bhi,
 
 template <int RJ, int KA>
 __global__ void __launch_bounds__(kSThreads, 1)
-    k_socs_synth_tc(const float2* __restrict__ T, const SocsGeom g, const float2* __restrict__ ty, int nsplit,
+    k_socs_synth_tc(const float2* __restrict__ T, const SocsGeom g, const float2* __restrict__ ty,
                     const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo,
                     const __grid_constant__ CUtensorMap tm_img, int nimg, int* __restrict__ err) {
   constexpr int J = 32 * RJ;
@@ -174,6 +175,8 @@ __global__ void __launch_bounds__(kSThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  dep_wait();
+  dep_launch();
 
   if (warp == kProdWarp) {
     // TMA producer (one lane): per N tile, for each K atom the hi unit then
@@ -376,22 +379,16 @@ __global__ void __launch_bounds__(kSThreads, 1)
       if (img != cur_img) {
         cur_img = img;
         if (tid == 0) s_bound = 0u;
-        const float2* Ti = T + (size_t)img * nsplit * tsz;
+        const float2* Ti = T + (size_t)img * tsz;
         // eight independent loads in flight per thread (the first tile of a
         // run waits on them)
         for (int i0 = tid; i0 < nty * tstr; i0 += 8 * 32 * kCW) {
           float2 v[8];
-          size_t o[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * 32 * kCW, ar = i / tstr, b = i - ar * tstr;
-            o[u] = (i < nty * tstr && b < ntx) ? (size_t)ar * ntx + b : SIZE_MAX;
-            v[u] = o[u] != SIZE_MAX ? __ldg(Ti + o[u]) : make_float2(0.f, 0.f);
+            v[u] = (i < nty * tstr && b < ntx) ? __ldg(Ti + (size_t)ar * ntx + b) : make_float2(0.f, 0.f);
           }
-          for (int p = 1; p < nsplit; ++p)
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (o[u] != SIZE_MAX) v[u] = cadd(v[u], __ldg(Ti + p * tsz + o[u]));
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * 32 * kCW;
@@ -527,7 +524,7 @@ int synth_tc_build_basis(const SocsGeom& g, void* bhi, void* blo, cudaStream_t s
 
 namespace {
 template <int RJ, int KA>
-int launch_synth(const SocsGeom& g, const float2* T, const float2* ty, int nsplit, const void* bhi, const void* blo,
+int launch_synth(const SocsGeom& g, const float2* T, const float2* ty, const void* bhi, const void* blo,
                  int nimg, float* images, int* err, cudaStream_t st) {
   const int Kp = 64 * KA;
   CUtensorMap mh, ml, mi;
@@ -553,7 +550,7 @@ int launch_synth(const SocsGeom& g, const float2* T, const float2* ty, int nspli
   const int tiles = nimg * (g.Ly / kRows);
   const int per = (tiles + sms - 1) / sms;
   const int grid = (tiles + per - 1) / per;
-  kern<<<grid, kSThreads, sm, st>>>(T, g, ty, nsplit, mh, ml, mi, nimg, err);
+  KL_CUDA_TRY(launch_dependent(kern, grid, kSThreads, sm, st, T, g, ty, mh, ml, mi, nimg, err));
   KL_CUDA_TRY(cudaGetLastError());
   return KL_OK;
 }
@@ -561,7 +558,7 @@ int launch_synth(const SocsGeom& g, const float2* T, const float2* ty, int nspli
 
 bool synth_tc_aligned(const float* images) { return (reinterpret_cast<uintptr_t>(images) & 15) == 0; }
 
-int synth_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int nsplit, const void* bhi,
+int synth_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, const void* bhi,
                     const void* blo, int nimg, float* images, int* err, cudaStream_t st) {
   if (nimg <= 0) return KL_OK;
   if (!synth_tc_supported(g) || !synth_tc_aligned(images)) {
@@ -569,12 +566,12 @@ int synth_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int ns
     return KL_ERR_UNSUPPORTED;
   }
   const int RJ = g.J / 32, KA = synth_ka(g);
-  if (RJ == 1 && KA == 1) return launch_synth<1, 1>(g, T, ty, nsplit, bhi, blo, nimg, images, err, st);
-  if (RJ == 1 && KA == 2) return launch_synth<1, 2>(g, T, ty, nsplit, bhi, blo, nimg, images, err, st);
-  if (RJ == 2 && KA == 1) return launch_synth<2, 1>(g, T, ty, nsplit, bhi, blo, nimg, images, err, st);
-  if (RJ == 2 && KA == 2) return launch_synth<2, 2>(g, T, ty, nsplit, bhi, blo, nimg, images, err, st);
-  if (RJ == 4 && KA == 1) return launch_synth<4, 1>(g, T, ty, nsplit, bhi, blo, nimg, images, err, st);
-  return launch_synth<4, 2>(g, T, ty, nsplit, bhi, blo, nimg, images, err, st);
+  if (RJ == 1 && KA == 1) return launch_synth<1, 1>(g, T, ty, bhi, blo, nimg, images, err, st);
+  if (RJ == 1 && KA == 2) return launch_synth<1, 2>(g, T, ty, bhi, blo, nimg, images, err, st);
+  if (RJ == 2 && KA == 1) return launch_synth<2, 1>(g, T, ty, bhi, blo, nimg, images, err, st);
+  if (RJ == 2 && KA == 2) return launch_synth<2, 2>(g, T, ty, bhi, blo, nimg, images, err, st);
+  if (RJ == 4 && KA == 1) return launch_synth<4, 1>(g, T, ty, bhi, blo, nimg, images, err, st);
+  return launch_synth<4, 2>(g, T, ty, bhi, blo, nimg, images, err, st);
 }
 
 }  // namespace kl

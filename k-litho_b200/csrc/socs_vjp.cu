@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_vjp_inverse(const float2* __res
                                                           const SocsGeom g,
                                                           const float2* __restrict__ tx,
                                                           const float2* __restrict__ ty,
-                                                          int nsplit, int nsets,
+                                                          int nsets,
                                                           const float* __restrict__ targets,
                                                           float alpha, float thr,
                                                           float* __restrict__ images,
@@ -66,13 +66,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_vjp_inverse(const float2* __res
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int s = blockIdx.x, img = blockIdx.y, clip = img / nsets;
   const size_t tsz = (size_t)g.nty * g.ntx;
-  const float2* Ti = T + (size_t)img * nsplit * tsz;
+  const float2* Ti = T + (size_t)img * tsz;
 
-  for (int i = threadIdx.x; i < (int)tsz; i += kThreads) {
-    float2 v = __ldg(Ti + i);
-    for (int p = 1; p < nsplit; ++p) v = cadd(v, __ldg(Ti + p * tsz + i));
-    Ts[i] = v;
-  }
+  for (int i = threadIdx.x; i < (int)tsz; i += kThreads) Ts[i] = __ldg(Ti + i);
   for (int i = threadIdx.x; i < NBM * V; i += kThreads) tw[i] = __ldg(tx + i);
   for (int i = threadIdx.x; i < g.nty; i += kThreads) ph[i] = __ldg(ty + (size_t)s * g.nty + i);
   for (int i = threadIdx.x; i < J * QP; i += kThreads) Qs[i] = make_float2(0.f, 0.f);
@@ -526,7 +522,7 @@ int check_launch(const char* what) {
 
 template <int P, int V, int NBM, int RJ>
 int launch_vinv(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T, int nimg,
-                int nsplit, int nsets, const float* targets, float alpha, float thr, float* images,
+                int nsets, const float* targets, float alpha, float thr, float* images,
                 double* loss, float2* gpart, cudaStream_t st) {
   constexpr int J = 32 * RJ;
   const size_t toff = (size_t)NBM * V + (size_t)J * (NBM + 1) + (size_t)J * NBM + (size_t)g.nty * g.ntx + g.nty;
@@ -534,7 +530,7 @@ int launch_vinv(const SocsGeom& g, const float2* tx, const float2* ty, const flo
   auto kern = k_vjp_inverse<P, V, NBM, RJ>;
   int rc = set_smem(kern, sm);
   if (rc) return rc;
-  kern<<<dim3(g.nS, nimg), kThreads, sm, st>>>(T, g, tx, ty, nsplit, nsets, targets, alpha, thr,
+  kern<<<dim3(g.nS, nimg), kThreads, sm, st>>>(T, g, tx, ty, nsets, targets, alpha, thr,
                                                  images, loss, gpart);
   return check_launch("k_vjp_inverse");
 }
@@ -564,13 +560,13 @@ size_t vjp_gpart_bytes(const SocsGeom& g, int nimg) {
 }
 
 int vjp_launch_inverse(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T,
-                       int nclips, int nsets, int nsplit, const float* targets, float alpha,
+                       int nclips, int nsets, const float* targets, float alpha,
                        float thr, float* images, double* loss, float2* gpart, cudaStream_t st) {
   if (nclips <= 0) return KL_OK;
   const int RJ = g.J / 32, nimg = nclips * nsets;
 #define KL_VINV(P_, V_, R_)                               \
   if (g.P == P_ && g.V == V_ && RJ == R_)               \
-    return launch_vinv<P_, V_, 32, R_>(g, tx, ty, T, nimg, nsplit, nsets, targets, alpha, thr, images, loss, gpart, st);
+    return launch_vinv<P_, V_, 32, R_>(g, tx, ty, T, nimg, nsets, targets, alpha, thr, images, loss, gpart, st);
   KL_VINV(8, 32, 1) KL_VINV(8, 32, 2) KL_VINV(16, 32, 1) KL_VINV(16, 32, 2)
   KL_VINV(32, 32, 1) KL_VINV(32, 32, 2) KL_VINV(32, 64, 1) KL_VINV(32, 64, 2)
   KL_VINV(8, 96, 1) KL_VINV(8, 96, 2) KL_VINV(16, 96, 1) KL_VINV(16, 96, 2)

@@ -105,7 +105,7 @@ __global__ void k_vjp_basis_t(int Lx, int ntx, __half* __restrict__ bhi, __half*
 
 template <int RJ>
 __global__ void __launch_bounds__(vThreads, 1)
-    k_vjp_synth_tc(const float2* __restrict__ T, const SocsGeom g, const float2* __restrict__ ty, int nsplit,
+    k_vjp_synth_tc(const float2* __restrict__ T, const SocsGeom g, const float2* __restrict__ ty,
                    int nsets, const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo,
                    const __grid_constant__ CUtensorMap tm_thi, const __grid_constant__ CUtensorMap tm_tlo,
                    const __grid_constant__ CUtensorMap tm_img, const __grid_constant__ CUtensorMap tm_tgt,
@@ -581,22 +581,16 @@ __global__ void __launch_bounds__(vThreads, 1)
       if (img != cur_img) {
         cur_img = img;
         if (tid == 0) s_bound = 0u;
-        const float2* Ti = T + (size_t)img * nsplit * tsz;
+        const float2* Ti = T + (size_t)img * tsz;
         // eight independent loads in flight per thread (the first tile of a
         // run waits on them)
         for (int i0 = tid; i0 < nty * tstr; i0 += 8 * 32 * vCW) {
           float2 v[8];
-          size_t o[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * 32 * vCW, ar = i / tstr, b = i - ar * tstr;
-            o[u] = (i < nty * tstr && b < ntx) ? (size_t)ar * ntx + b : SIZE_MAX;
-            v[u] = o[u] != SIZE_MAX ? __ldg(Ti + o[u]) : make_float2(0.f, 0.f);
+            v[u] = (i < nty * tstr && b < ntx) ? __ldg(Ti + (size_t)ar * ntx + b) : make_float2(0.f, 0.f);
           }
-          for (int p = 1; p < nsplit; ++p)
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-              if (o[u] != SIZE_MAX) v[u] = cadd(v[u], __ldg(Ti + p * tsz + o[u]));
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * 32 * vCW;
@@ -724,7 +718,7 @@ int vjp_tc_build_basis_t(const SocsGeom& g, void* thi, void* tlo, cudaStream_t s
 
 namespace {
 template <int RJ>
-int launch_vjp_tc(const SocsGeom& g, const float2* T, const float2* ty, int nclips, int nsets, int nsplit,
+int launch_vjp_tc(const SocsGeom& g, const float2* T, const float2* ty, int nclips, int nsets,
                   const void* bhi, const void* blo, const void* thi, const void* tlo, const float* targets,
                   float alpha, float thr, float* images, double* loss, float2* gpart, int* err, cudaStream_t st) {
   const int nimg = nclips * nsets;
@@ -761,14 +755,14 @@ int launch_vjp_tc(const SocsGeom& g, const float2* T, const float2* ty, int ncli
   const int tiles = nimg * (g.Ly / vRows);
   const int per = (tiles + sms - 1) / sms;
   const int grid = (tiles + per - 1) / per;
-  kern<<<grid, vThreads, sm, st>>>(T, g, ty, nsplit, nsets, mh, ml, mth, mtl, mi, mt, images ? 1 : 0, alpha, thr,
+  kern<<<grid, vThreads, sm, st>>>(T, g, ty, nsets, mh, ml, mth, mtl, mi, mt, images ? 1 : 0, alpha, thr,
                                    gscale, nimg, loss, gpart, err);
   KL_CUDA_TRY(cudaGetLastError());
   return KL_OK;
 }
 }  // namespace
 
-int vjp_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int nclips, int nsets, int nsplit,
+int vjp_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int nclips, int nsets,
                   const void* bhi, const void* blo, const void* thi, const void* tlo, const float* targets,
                   float alpha, float thr, float* images, double* loss, float2* gpart, int* err, cudaStream_t st) {
   if (nclips <= 0) return KL_OK;
@@ -777,9 +771,9 @@ int vjp_tc_launch(const SocsGeom& g, const float2* T, const float2* ty, int ncli
     return KL_ERR_UNSUPPORTED;
   }
   if (g.J == 32)
-    return launch_vjp_tc<1>(g, T, ty, nclips, nsets, nsplit, bhi, blo, thi, tlo, targets, alpha, thr, images, loss,
+    return launch_vjp_tc<1>(g, T, ty, nclips, nsets, bhi, blo, thi, tlo, targets, alpha, thr, images, loss,
                             gpart, err, st);
-  return launch_vjp_tc<2>(g, T, ty, nclips, nsets, nsplit, bhi, blo, thi, tlo, targets, alpha, thr, images, loss,
+  return launch_vjp_tc<2>(g, T, ty, nclips, nsets, bhi, blo, thi, tlo, targets, alpha, thr, images, loss,
                           gpart, err, st);
 }
 
