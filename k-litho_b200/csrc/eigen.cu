@@ -145,6 +145,105 @@ int zgemm(const void* A, int lda, const void* Bm, int ldb, double2* C, int ldc, 
   return KL_OK;
 }
 
+// Tall or small products of the subspace iteration: C (M x N, N <= 64) with k split
+// over the grid.  The 32 x 32 tiles above give such shapes a handful of CTAs (8 for
+// a 36 x 36 Gram matrix of 729 rows, 55 us) and an almost empty second tile; here a
+// CTA has 16 rows and every column (a multiple of 16, Q outputs per thread), the
+// next k step is loaded while one is multiplied, and as many k slices run as fill
+// the SMs twice.  The slice that finishes last adds them up in order.
+constexpr int kSkinnyMaxN = 64;
+constexpr int kSkinnyTiles = 148;  // 16-row tiles of a product whose k is split
+
+template <int MODE, int Q>
+__global__ void __launch_bounds__(256) k_zskinny(const void* __restrict__ A, int lda, const void* __restrict__ Bm,
+                                                 int ldb, double2* __restrict__ C, int ldc, int M, int N, int K,
+                                                 double2* __restrict__ part, int* __restrict__ cnt) {
+  constexpr int TK = 16, TN = 16 * Q;
+  constexpr bool kByRow = MODE == G_AY || MODE == G_DX || MODE == G_FX || MODE == G_NN;  // A contiguous in k
+  __shared__ double2 sa[TK][17];
+  __shared__ double2 sb[TK][TN];
+  __shared__ int s_last;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4, m0 = blockIdx.x * 16;
+  const int nz = gridDim.y, kc = ((K + nz - 1) / nz + TK - 1) / TK * TK;
+  const int kbeg = min(K, (int)blockIdx.y * kc), kend = min(K, kbeg + kc);
+  const double2 zero = make_double2(0.0, 0.0);
+  const int am = m0 + (kByRow ? ty : tx), ak = kByRow ? tx : ty;
+  double2 ra, rb[Q];
+  auto fetch = [&](int k0) {
+    ra = am < M && k0 + ak < kend ? load_a<MODE>(A, lda, am, k0 + ak) : zero;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int e = t + 256 * q, k = k0 + e / TN, n = e % TN;
+      rb[q] = n < N && k < kend ? load_b<MODE>(Bm, ldb, k, n) : zero;
+    }
+  };
+  double2 acc[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) acc[q] = zero;
+  if (kbeg < kend) fetch(kbeg);
+  for (int k0 = kbeg; k0 < kend; k0 += TK) {
+    sa[ak][kByRow ? ty : tx] = ra;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int e = t + 256 * q;
+      sb[e / TN][e % TN] = rb[q];
+    }
+    __syncthreads();
+    if (k0 + TK < kend) fetch(k0 + TK);
+#pragma unroll
+    for (int k = 0; k < TK; ++k) {
+      const double2 a = sa[k][ty];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) acc[q] = zfma(a, sb[k][tx + 16 * q], acc[q]);
+    }
+    __syncthreads();
+  }
+  if (nz > 1) {
+    double2* p = part + (size_t)blockIdx.x * nz * 16 * TN + (size_t)ty * TN + tx;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) p[(size_t)blockIdx.y * 16 * TN + 16 * q] = acc[q];
+    __threadfence();
+    __syncthreads();
+    if (t == 0) s_last = atomicAdd(cnt + blockIdx.x, 1) == nz - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (t == 0) cnt[blockIdx.x] = 0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) acc[q] = zero;
+#pragma unroll 4
+    for (int z = 0; z < nz; ++z)
+#pragma unroll
+      for (int q = 0; q < Q; ++q) acc[q] = zadd(acc[q], __ldcg(p + (size_t)z * 16 * TN + 16 * q));
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (m0 + ty < M && tx + 16 * q < N) C[(size_t)(m0 + ty) * ldc + tx + 16 * q] = acc[q];
+}
+
+// k slices of a skinny product, and whether its shape takes that kernel: at most
+// 64 columns and too few 32 x 32 tiles to fill the SMs twice
+int skinny_slices(int M, int K) { return std::max(1, std::min(2 * 148 / ((M + 15) / 16), K / 32)); }
+bool skinny_shape(int M, int N) { return N <= kSkinnyMaxN && ((M + 31) / 32) * ((N + 31) / 32) < 296; }
+
+// zgemm of the iteration; part / cnt: skinny_part_elems elements, kSkinnyTiles
+// counters (zero, left zero)
+size_t skinny_part_elems(int N) { return (size_t)(2 * 148) * 16 * ((N + 15) / 16 * 16); }
+template <int MODE>
+int zgemm_iter(const void* A, int lda, const void* Bm, int ldb, double2* C, int ldc, int M, int N, int K,
+               double2* part, int* cnt, cudaStream_t st) {
+  if (!skinny_shape(M, N)) return zgemm<MODE>(A, lda, Bm, ldb, C, ldc, M, N, K, st);
+  const dim3 grid((M + 15) / 16, skinny_slices(M, K));
+  switch ((N + 15) / 16) {
+    case 1: k_zskinny<MODE, 1><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, C, ldc, M, N, K, part, cnt); break;
+    case 2: k_zskinny<MODE, 2><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, C, ldc, M, N, K, part, cnt); break;
+    case 3: k_zskinny<MODE, 3><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, C, ldc, M, N, K, part, cnt); break;
+    default: k_zskinny<MODE, 4><<<grid, 256, 0, st>>>(A, lda, Bm, ldb, C, ldc, M, N, K, part, cnt); break;
+  }
+  KL_CUDA_TRY(cudaGetLastError());
+  return KL_OK;
+}
+
 // deterministic start block, entries uniform in [-1, 1] + i[-1, 1]
 __global__ void k_rand_block(double2* X, int N, int B, uint64_t seed) {
   const size_t n = (size_t)N * B;
@@ -218,6 +317,119 @@ __global__ void __launch_bounds__(256) k_chol_inv(const double2* __restrict__ G,
     }
   }
   if (threadIdx.x == 0 && s_bad) status[0] = 1;
+}
+
+// The same for B <= 16 NB <= 64 with the matrix in registers: thread (ty, tx) of 16 x 16
+// holds entries (ty + 16 a, tx + 16 b).  Latency of one CTA: a step is one barrier, a
+// row exchanged through shared memory, and NB^2 independent updates; rows stay
+// unscaled (L D L^H) until the end.  36 columns took 81 us in the kernel above, and 57
+// us at 48 with its updates on shared memory; here 11.
+template <int NB>
+__global__ void __launch_bounds__(256) k_chol_inv_reg(const double2* __restrict__ G, int B, double rel_shift,
+                                                      double2* __restrict__ Rinv, int* __restrict__ status) {
+  constexpr int NP = 16 * NB;
+  extern __shared__ double2 sm[];
+  double2(*U)[NP + 1] = reinterpret_cast<double2(*)[NP + 1]>(sm);  // [NP][NP + 1] the factor's rows, unscaled
+  __shared__ double2 row[2][NP];
+  __shared__ double s_max[8], s_q[NP];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 r[NB][NB];
+  double mx = 0.0;
+#pragma unroll
+  for (int a = 0; a < NB; ++a)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int i = ty + 16 * a, l = tx + 16 * b;
+      r[a][b] = i < B && l < B ? G[(size_t)i * B + l] : zero;
+      if (i == l) mx = fmax(mx, r[a][b].x);
+    }
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  double shift = 0.0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) shift = fmax(shift, s_max[w]);
+  shift *= rel_shift;
+#pragma unroll
+  for (int a = 0; a < NB; ++a)
+    if (ty == tx) r[a][a].x += shift;
+  bool bad = false;
+  // r[i][l] -= conj(r[j][i]) r[j][l] / r[j][j], j < i <= l (the lower part is not used)
+#pragma unroll
+  for (int aj = 0; aj < NB; ++aj) {
+#pragma unroll 1
+    for (int jj = 0; jj < 16; ++jj) {
+      const int j = 16 * aj + jj;
+      if (j >= B) break;
+      if (ty == jj) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          row[j & 1][tx + 16 * b] = r[aj][b];
+          U[j][tx + 16 * b] = r[aj][b];
+        }
+      }
+      __syncthreads();
+      const double d2 = row[j & 1][j].x;
+      const double inv = d2 > 0.0 ? 1.0 / d2 : 0.0;
+      bad = bad || !(d2 > 0.0);
+      if (threadIdx.x == 0) s_q[j] = inv;
+      double2 y[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) y[b] = row[j & 1][tx + 16 * b];
+#pragma unroll
+      for (int a = aj; a < NB; ++a) {
+        const double2 x = row[j & 1][ty + 16 * a];
+        const double2 f = ty + 16 * a > j ? make_double2(-x.x * inv, x.y * inv) : zero;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) r[a][b] = zfma(f, y[b], r[a][b]);
+      }
+    }
+  }
+  __syncthreads();
+  // row i of the factor is U[i][:] / sqrt(pivot_i): its inverse X from the last row up,
+  // X[i][:] = e_i / sqrt(pivot_i) - sum_{l > i} U[i][l] / pivot_i X[l][:]
+#pragma unroll
+  for (int a = 0; a < NB; ++a)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int i = ty + 16 * a, c = tx + 16 * b;
+      r[a][b] = make_double2(i == c && i < B ? sqrt(s_q[i]) : 0.0, 0.0);
+    }
+  double q[NB];
+#pragma unroll
+  for (int a = 0; a < NB; ++a) q[a] = ty + 16 * a < B ? s_q[ty + 16 * a] : 0.0;
+#pragma unroll
+  for (int al = NB - 1; al >= 0; --al) {
+#pragma unroll 1
+    for (int ll = 15; ll >= 0; --ll) {
+      const int l = 16 * al + ll;
+      if (l >= B) continue;
+      if (ty == ll) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) row[l & 1][tx + 16 * b] = r[al][b];
+      }
+      __syncthreads();
+      double2 y[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) y[b] = row[l & 1][tx + 16 * b];
+#pragma unroll
+      for (int a = 0; a <= al; ++a) {
+        const double2 x = U[ty + 16 * a][l];
+        const double2 f = ty + 16 * a < l ? make_double2(-x.x * q[a], -x.y * q[a]) : zero;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) r[a][b] = zfma(f, y[b], r[a][b]);
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < NB; ++a)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int i = ty + 16 * a, c = tx + 16 * b;
+      if (i < B && c < B) Rinv[(size_t)i * B + c] = r[a][b];
+    }
+  if (threadIdx.x == 0 && bad) status[0] = 1;
 }
 
 // Hermitian eigensolve H = Q diag(w) Q^H by cyclic Jacobi with the
@@ -1116,6 +1328,9 @@ struct Workspace {
   double4* rot = nullptr;
   double* w = nullptr;
   int *status = nullptr, *jst = nullptr;
+  double2* part = nullptr;  // k slices of the skinny products, and their counters
+  int* cnt = nullptr;
+  double* res = nullptr;  // squared residuals of the Ritz pairs
   cudaStream_t st = nullptr;
   std::vector<void*> owned;
   template <typename T>
@@ -1269,17 +1484,38 @@ size_t jacobi_log_elems(int B) {  // double4 units
   return (size_t)kJacobiMaxSweeps * (Bp - 1) * (Bp / 2) + 1;
 }
 
-// X (N x B) <- orth(X) by CholeskyQR2; the first pass shifted for safety
-int cholqr2(double2* X, int N, int B, Workspace& ws, cudaStream_t st) {
-  for (int pass = 0; pass < 2; ++pass) {
-    int rc = zgemm<G_HH>(X, B, X, B, ws.G, B, B, B, N, st);
+template <int NB>
+int chol_inv_reg(const double2* G, int B, double rel_shift, double2* Rinv, int* status, cudaStream_t st) {
+  constexpr size_t sm = sizeof(double2) * 16 * NB * (16 * NB + 1);
+  if (sm > 40 * 1024)
+    KL_CUDA_TRY(cudaFuncSetAttribute(k_chol_inv_reg<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  k_chol_inv_reg<NB><<<1, 256, sm, st>>>(G, B, rel_shift, Rinv, status);
+  KL_CUDA_TRY(cudaGetLastError());
+  return KL_OK;
+}
+
+int chol_inv(const double2* G, int B, double rel_shift, double2* Rinv, int* status, cudaStream_t st) {
+  switch ((B + 15) / 16) {
+    case 1: return chol_inv_reg<1>(G, B, rel_shift, Rinv, status, st);
+    case 2: return chol_inv_reg<2>(G, B, rel_shift, Rinv, status, st);
+    case 3: return chol_inv_reg<3>(G, B, rel_shift, Rinv, status, st);
+    case 4: return chol_inv_reg<4>(G, B, rel_shift, Rinv, status, st);
+  }
+  k_chol_inv<<<1, 256, sizeof(double2) * (size_t)B * B, st>>>(G, B, rel_shift, Rinv, status);
+  KL_CUDA_TRY(cudaGetLastError());
+  return KL_OK;
+}
+
+// ws.X (N x B) <- orth(ws.X) by Cholesky QR, twice unless one pass will do; the
+// first pass shifted for safety
+int cholqr(int N, int B, int passes, Workspace& ws, cudaStream_t st) {
+  for (int pass = 0; pass < passes; ++pass) {
+    int rc = zgemm_iter<G_HH>(ws.X, B, ws.X, B, ws.G, B, B, B, N, ws.part, ws.cnt, st);
     if (rc) return rc;
-    k_chol_inv<<<1, 256, sizeof(double2) * (size_t)B * B, st>>>(ws.G, B, pass == 0 ? 1e-14 : 0.0,
-                                                                ws.Rinv, ws.status);
-    KL_CUDA_TRY(cudaGetLastError());
-    rc = zgemm<G_NN>(X, B, ws.Rinv, B, ws.W, B, N, B, B, st);
+    if ((rc = chol_inv(ws.G, B, pass == 0 ? 1e-14 : 0.0, ws.Rinv, ws.status, st))) return rc;
+    rc = zgemm_iter<G_NN>(ws.X, B, ws.Rinv, B, ws.W, B, N, B, B, ws.part, ws.cnt, st);
     if (rc) return rc;
-    KL_CUDA_TRY(cudaMemcpyAsync(X, ws.W, sizeof(double2) * (size_t)N * B, cudaMemcpyDeviceToDevice, st));
+    std::swap(ws.X, ws.W);
   }
   return KL_OK;
 }
@@ -1336,7 +1572,27 @@ int jacobi(double2* H, int B, double4* rot, int* jst, double2* Q, double* w, cud
   return jacobi_batch({JacobiJob{H, rot, Q, w, jst, B}}, st);
 }
 
-// Generic driver.  apply(X, W): W = TCC X (N x B); project(X, H): H = X^H TCC X (B x B).
+// res[k] = |W[:, k] - w[k] X[:, k]|^2, one CTA per column
+__global__ void __launch_bounds__(128) k_ritz_residual(const double2* __restrict__ X, const double2* __restrict__ W,
+                                                       const double* __restrict__ w, int N, int B,
+                                                       double* __restrict__ res) {
+  const int k = blockIdx.x;
+  const double wk = w[k];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < N; i += 128) {
+    const double2 x = X[(size_t)i * B + k], y = W[(size_t)i * B + k];
+    const double a = fma(-wk, x.x, y.x), b = fma(-wk, x.y, y.y);
+    s = fma(a, a, fma(b, b, s));
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __shared__ double part[4];
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) res[k] = part[0] + part[1] + part[2] + part[3];
+}
+
+// Generic driver.  apply(ws, X, W): W = TCC X (N x B); project(ws, X, H): H = X^H TCC X
+// (B x B).
 template <typename Apply, typename Project>
 int subspace_iteration(int N, const EigenOptions& opt, int B, Apply apply, Project project,
                        double2* U, double* evals, EigenResult* res, cudaStream_t st) {
@@ -1348,64 +1604,95 @@ int subspace_iteration(int N, const EigenOptions& opt, int B, Apply apply, Proje
       (arc = ws.get(&ws.G, (size_t)B * B)) || (arc = ws.get(&ws.Rinv, (size_t)B * B)) ||
       (arc = ws.get(&ws.Q, (size_t)B * B)) || (arc = ws.get(&ws.rot, jacobi_log_elems(B))) ||
       (arc = ws.get(&ws.jst, (size_t)B + 1)) || (arc = ws.get(&ws.w, (size_t)B)) ||
-      (arc = ws.get(&ws.status, 1)))
+      (arc = ws.get(&ws.part, skinny_part_elems(std::min(B, kSkinnyMaxN)))) ||
+      (arc = ws.get(&ws.cnt, kSkinnyTiles)) || (arc = ws.get(&ws.res, (size_t)K)) || (arc = ws.get(&ws.status, 1)))
     return arc;
   const size_t sm_chol = sizeof(double2) * (size_t)B * B;
   if (sm_chol > 48 * 1024)
     KL_CUDA_TRY(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_chol));
   KL_CUDA_TRY(cudaMemsetAsync(ws.status, 0, sizeof(int), st));
+  KL_CUDA_TRY(cudaMemsetAsync(ws.cnt, 0, sizeof(int) * kSkinnyTiles, st));
   k_rand_block<<<256, 256, 0, st>>>(ws.X, N, B, opt.seed);
   KL_CUDA_TRY(cudaGetLastError());
   int rc;
   // one power step on the random block, then orthonormalise
-  if ((rc = apply(ws.X, ws.W))) return rc;
-  KL_CUDA_TRY(cudaMemcpyAsync(ws.X, ws.W, sizeof(double2) * (size_t)N * B, cudaMemcpyDeviceToDevice, st));
-  if ((rc = cholqr2(ws.X, N, B, ws, st))) return rc;
+  if ((rc = apply(ws, ws.X, ws.W))) return rc;
+  std::swap(ws.X, ws.W);
+  if ((rc = cholqr(N, B, 2, ws, st))) return rc;
 
-  std::vector<double> prev(K, 0.0), cur(B, 0.0);
-  int it = 0;
-  double change = 1.0;
-  const int check_every = 2;
-  bool converged = false;
+  // A check rotates the block to its Ritz vectors and takes their residuals from the
+  // next product, W = TCC X.  A Ritz value is off by residual^2 / gap at most (gap: to
+  // the block's smallest, beyond which lies what is not in it), and that falls by
+  // (w_B / w_K)^2 per iteration, so the first check says where the last one belongs
+  // (each is a Jacobi solve on one SM, 0.35 ms at B = 48; an iteration is 50 us).
+  // Residuals of 1e-14 of the largest eigenvalue are rounding.
+  std::vector<double> cur(B, 0.0), rs(K, 0.0);
+  int it = 0, next = std::min(3, opt.max_iter);
+  double error = 1.0;
+  bool converged = false, one_pass = false, may_skip = false, skipped = false;
   for (it = 1; it <= opt.max_iter; ++it) {
-    if (it % check_every == 0) {
-      if ((rc = project(ws.X, ws.G))) return rc;
+    const bool check = it == next;
+    if (check) {
+      if ((rc = project(ws, ws.X, ws.G))) return rc;
       if ((rc = jacobi(ws.G, B, ws.rot, ws.jst, ws.Q, ws.w, st))) return rc;
+      // continue from the Ritz basis: the next projected matrix is then nearly
+      // diagonal and its Jacobi solve takes a few sweeps
+      if ((rc = zgemm_iter<G_NN>(ws.X, B, ws.Q, B, ws.W, B, N, B, B, ws.part, ws.cnt, st))) return rc;
+      std::swap(ws.X, ws.W);
+    }
+    if ((rc = apply(ws, ws.X, ws.W))) return rc;
+    if (check) {
+      k_ritz_residual<<<K, 128, 0, st>>>(ws.X, ws.W, ws.w, N, B, ws.res);
+      KL_CUDA_TRY(cudaGetLastError());
       int jsteps = 0;
       KL_CUDA_TRY(cudaMemcpyAsync(cur.data(), ws.w, sizeof(double) * B, cudaMemcpyDeviceToHost, st));
+      KL_CUDA_TRY(cudaMemcpyAsync(rs.data(), ws.res, sizeof(double) * K, cudaMemcpyDeviceToHost, st));
       KL_CUDA_TRY(cudaMemcpyAsync(&jsteps, ws.jst, sizeof(int), cudaMemcpyDeviceToHost, st));
       KL_CUDA_TRY(cudaStreamSynchronize(st));
       if (jsteps < 0) {
         set_error("subspace iteration: the cluster Jacobi eigensolve timed out exchanging rotations");
         return KL_ERR_CUDA;
       }
-      change = 0.0;
+      error = 0.0;
       for (int k = 0; k < K; ++k) {
         const double den = std::max(std::fabs(cur[k]), 1e-300 + std::fabs(cur[0]) * 1e-16);
-        change = std::max(change, std::fabs(cur[k] - prev[k]) / den);
-        prev[k] = cur[k];
+        const double gap = std::max(cur[k] - cur[B - 1], 0.05 * den);
+        if (!(rs[k] <= 1e-28 * cur[0] * cur[0])) error = std::max(error, rs[k] / (gap * den));  // rs: squared
       }
-      if (change < opt.tol) {
+      if (error < opt.tol) {
         converged = true;
         break;
       }
-      // continue from the Ritz basis: the next projected matrix is then nearly
-      // diagonal and its Jacobi solve takes a few sweeps
-      if ((rc = zgemm<G_NN>(ws.X, B, ws.Q, B, ws.W, B, N, B, B, st))) return rc;
-      KL_CUDA_TRY(cudaMemcpyAsync(ws.X, ws.W, sizeof(double2) * (size_t)N * B, cudaMemcpyDeviceToDevice, st));
+      int step = 2;
+      if (cur[B - 1] > 0.0 && cur[B - 1] < cur[K - 1]) {
+        const double rate = 2.0 * std::log(cur[B - 1] / cur[K - 1]);
+        step = std::max(2, std::min(24, 1 + (int)std::ceil(std::log(opt.tol / error) / rate)));
+      }
+      next = std::min(it + step, std::max(it + 1, opt.max_iter));
+      // The basis need be orthonormal only for the checks.  Between them one pass of
+      // Cholesky QR keeps it well conditioned if the block's spectrum is not steep
+      // (condition w_0 / w_B after a product), and every other iteration can do without
+      const double steep = cur[B - 1] > 0.0 ? cur[0] / cur[B - 1] : 1e300;
+      one_pass = steep < 1e5;
+      may_skip = steep < 1e3;
+      skipped = false;
     }
-    if ((rc = apply(ws.X, ws.W))) return rc;
-    KL_CUDA_TRY(cudaMemcpyAsync(ws.X, ws.W, sizeof(double2) * (size_t)N * B, cudaMemcpyDeviceToDevice, st));
-    if ((rc = cholqr2(ws.X, N, B, ws, st))) return rc;
+    std::swap(ws.X, ws.W);
+    if (may_skip && !skipped && it + 2 < next) {
+      skipped = true;
+      continue;
+    }
+    skipped = false;
+    if ((rc = cholqr(N, B, one_pass && it + 1 != next ? 1 : 2, ws, st))) return rc;
   }
-  // final Rayleigh-Ritz on the current block (G holds the eigvecs in Q)
+  // U = the first K Ritz vectors (N x K, row-major), eigenvalues
   if (!converged) {
-    if ((rc = project(ws.X, ws.G))) return rc;
+    if ((rc = project(ws, ws.X, ws.G))) return rc;
     if ((rc = jacobi(ws.G, B, ws.rot, ws.jst, ws.Q, ws.w, st))) return rc;
+    if ((rc = zgemm_iter<G_NN>(ws.X, B, ws.Q, B, ws.W, B, N, B, B, ws.part, ws.cnt, st))) return rc;
+    std::swap(ws.X, ws.W);
   }
-  // U = X Q[:, :K] (N x K, row-major), eigenvalues
-  if ((rc = zgemm<G_NN>(ws.X, B, ws.Q, B, ws.W, B, N, B, B, st))) return rc;
-  KL_CUDA_TRY(cudaMemcpy2DAsync(U, sizeof(double2) * K, ws.W, sizeof(double2) * B, sizeof(double2) * K, N,
+  KL_CUDA_TRY(cudaMemcpy2DAsync(U, sizeof(double2) * K, ws.X, sizeof(double2) * B, sizeof(double2) * K, N,
                                 cudaMemcpyDeviceToDevice, st));
   KL_CUDA_TRY(cudaMemcpyAsync(evals, ws.w, sizeof(double) * K, cudaMemcpyDeviceToDevice, st));
   int status = 0;
@@ -1413,10 +1700,10 @@ int subspace_iteration(int N, const EigenOptions& opt, int B, Apply apply, Proje
   KL_CUDA_TRY(cudaStreamSynchronize(st));
   if (res) {
     res->iterations = std::min(it, opt.max_iter);
-    res->residual = change;
+    res->residual = error;
   }
-  if (!converged && change >= opt.tol) {
-    set_error("subspace iteration did not converge: relative Ritz change " + std::to_string(change) +
+  if (!converged) {
+    set_error("subspace iteration did not converge: relative Ritz error " + std::to_string(error) +
               " after " + std::to_string(opt.max_iter) + " iterations");
     return KL_ERR_NOT_CONVERGED;
   }
@@ -1565,15 +1852,15 @@ int eig_topk_factor(const float2* A, int N, int S, const EigenOptions& opt, doub
   KL_CHECK_ARG(opt.K <= B, "eig_topk_factor: K exceeds the block size");
   double2* Z = nullptr;
   if (int arc = scratch_alloc((void**)&Z, sizeof(double2) * (size_t)S * B, st, "eigen workspace")) return arc;
-  auto apply = [&](double2* X, double2* W) -> int {
-    int rc = zgemm<G_AHX>(A, S, X, B, Z, B, S, B, N, st);  // Z = A^H X
+  auto apply = [&](Workspace& ws, double2* X, double2* W) -> int {
+    int rc = zgemm_iter<G_AHX>(A, S, X, B, Z, B, S, B, N, ws.part, ws.cnt, st);  // Z = A^H X
     if (rc) return rc;
-    return zgemm<G_AY>(A, S, Z, B, W, B, N, B, S, st);      // W = A Z
+    return zgemm_iter<G_AY>(A, S, Z, B, W, B, N, B, S, ws.part, ws.cnt, st);      // W = A Z
   };
-  auto project = [&](double2* X, double2* H) -> int {
-    int rc = zgemm<G_AHX>(A, S, X, B, Z, B, S, B, N, st);  // Z = A^H X
+  auto project = [&](Workspace& ws, double2* X, double2* H) -> int {
+    int rc = zgemm_iter<G_AHX>(A, S, X, B, Z, B, S, B, N, ws.part, ws.cnt, st);  // Z = A^H X
     if (rc) return rc;
-    return zgemm<G_HH>(Z, B, Z, B, H, B, B, B, S, st);      // H = Z^H Z
+    return zgemm_iter<G_HH>(Z, B, Z, B, H, B, B, B, S, ws.part, ws.cnt, st);      // H = Z^H Z
   };
   int rc = subspace_iteration(N, opt, B, apply, project, U, evals, res, st);
   scratch_free(Z, st);
@@ -1602,13 +1889,13 @@ int eig_topk_dense(const double2* tcc, int N, const EigenOptions& opt, double2* 
   const int B = block_size(opt, N, N);
   double2* Wt = nullptr;
   if (int arc = scratch_alloc((void**)&Wt, sizeof(double2) * (size_t)N * B, st, "eigen workspace")) return arc;
-  auto apply = [&](double2* X, double2* W) -> int {
-    return zgemm<G_DX>(tcc, N, X, B, W, B, N, B, N, st);
+  auto apply = [&](Workspace& ws, double2* X, double2* W) -> int {
+    return zgemm_iter<G_DX>(tcc, N, X, B, W, B, N, B, N, ws.part, ws.cnt, st);
   };
-  auto project = [&](double2* X, double2* H) -> int {
-    int rc = zgemm<G_DX>(tcc, N, X, B, Wt, B, N, B, N, st);
+  auto project = [&](Workspace& ws, double2* X, double2* H) -> int {
+    int rc = zgemm_iter<G_DX>(tcc, N, X, B, Wt, B, N, B, N, ws.part, ws.cnt, st);
     if (rc) return rc;
-    return zgemm<G_HH>(X, B, Wt, B, H, B, B, B, N, st);
+    return zgemm_iter<G_HH>(X, B, Wt, B, H, B, B, B, N, ws.part, ws.cnt, st);
   };
   int rc = subspace_iteration(N, opt, B, apply, project, U, evals, res, st);
   scratch_free(Wt, st);
@@ -1621,13 +1908,13 @@ int eig_topk_dense_c64(const float2* tcc, int N, const EigenOptions& opt, double
   const int B = block_size(opt, N, N);
   double2* Wt = nullptr;
   if (int arc = scratch_alloc((void**)&Wt, sizeof(double2) * (size_t)N * B, st, "eigen workspace")) return arc;
-  auto apply = [&](double2* X, double2* W) -> int {
-    return zgemm<G_FX>(tcc, N, X, B, W, B, N, B, N, st);
+  auto apply = [&](Workspace& ws, double2* X, double2* W) -> int {
+    return zgemm_iter<G_FX>(tcc, N, X, B, W, B, N, B, N, ws.part, ws.cnt, st);
   };
-  auto project = [&](double2* X, double2* H) -> int {
-    int rc = zgemm<G_FX>(tcc, N, X, B, Wt, B, N, B, N, st);
+  auto project = [&](Workspace& ws, double2* X, double2* H) -> int {
+    int rc = zgemm_iter<G_FX>(tcc, N, X, B, Wt, B, N, B, N, ws.part, ws.cnt, st);
     if (rc) return rc;
-    return zgemm<G_HH>(X, B, Wt, B, H, B, B, B, N, st);
+    return zgemm_iter<G_HH>(X, B, Wt, B, H, B, B, B, N, ws.part, ws.cnt, st);
   };
   int rc = subspace_iteration(N, opt, B, apply, project, U, evals, res, st);
   scratch_free(Wt, st);

@@ -77,7 +77,7 @@ struct EigenOptions {
 struct EigenResult {
   int iterations;   // subspace iterations; Jacobi sweeps of a one-step Gram solve (1 when it
                     // ran the tridiagonal solver)
-  double residual;  // max relative Ritz-value change at the last check
+  double residual;  // bound of the relative error of the Ritz values at the last check
 };
 
 // One top-K problem on a TCC factor A (N x S), for the batched solver.

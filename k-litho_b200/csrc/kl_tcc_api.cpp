@@ -273,7 +273,10 @@ struct TopkBuffers {
 kl::EigenOptions topk_options(int K, int block) {
   kl::EigenOptions opt;
   opt.K = K;
-  opt.B = block > 0 ? block : std::min(K + std::max(16, K / 2), std::max(K, 2 * K));
+  // automatic block: a wider one converges in fewer iterations, and up to 64
+  // columns the products cost the same (20 iterations at 36 columns, 14 at 48 for
+  // 24 kernels of the annular source)
+  opt.B = block > 0 ? block : std::min(K + std::max(K <= 40 ? 24 : 16, K / 2), std::max(K, 2 * K));
   opt.max_iter = 400;
   opt.tol = 1e-13;
   opt.seed = 0x6b6c697468ull;
