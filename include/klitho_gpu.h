@@ -165,6 +165,11 @@ int kl_socs_plan_status(kl_socs_plan plan);
 int kl_socs_set_kernels(kl_socs_plan plan, int set, const float* krn_re_host,
                         const float* krn_im_host, const float* scales_host);
 
+/* kl_socs_set_kernels with the kernels as interleaved complex64 (re, im pairs:
+ * nk x N x 2 floats, e.g. kl_topk_eig_c64's output): copied to the device as
+ * they are. */
+int kl_socs_set_kernels_c64(kl_socs_plan plan, int set, const float* krn_host, const float* scales_host);
+
 /* images_dev[c][s] (nclips x nsets x Ly x Lx float32) from masks_dev
  * (nclips x Ly x Lx float32, already embedded in the period as createMask
  * does).  Stream-ordered. */

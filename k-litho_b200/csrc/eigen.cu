@@ -1742,7 +1742,7 @@ __global__ void k_ritz_scale(const double2* __restrict__ Q, int ldq, const doubl
 // cluster reduction handles (64 .. 256) take the tridiagonal solver
 // (eig_tridiag.cu), smaller ones Jacobi on one CTA; all problems of a path are
 // solved in one batch of launches.
-int eig_topk_gram(const std::vector<FactorProblem>& pr, cudaStream_t st) {
+int eig_topk_gram(const std::vector<FactorProblem>& pr, cudaStream_t st, const std::function<void()>& meanwhile) {
   const size_t n = pr.size();
   std::vector<Workspace> ws(n);
   std::vector<JacobiJob> jobs;
@@ -1797,11 +1797,14 @@ int eig_topk_gram(const std::vector<FactorProblem>& pr, cudaStream_t st) {
   std::vector<int> nsteps(n, 0), gerr(n, 0);
   for (size_t i = 0; i < n; ++i) {
     const int S = pr[i].S, K = pr[i].K;
-    if (ws[i].status) KL_CUDA_TRY(cudaMemcpyAsync(&gerr[i], ws[i].status, sizeof(int), cudaMemcpyDeviceToHost, st));
     k_ritz_scale<<<(S * K + 255) / 256, 256, 0, st>>>(ws[i].Q, S, ws[i].w, S, K, ws[i].W);
     KL_CUDA_TRY(cudaGetLastError());
     if ((rc = zgemm<G_AY>(pr[i].A, S, ws[i].W, K, pr[i].U, K, pr[i].N, K, S, st))) return rc;
     KL_CUDA_TRY(cudaMemcpyAsync(pr[i].evals, ws[i].w, sizeof(double) * K, cudaMemcpyDeviceToDevice, st));
+  }
+  if (meanwhile) meanwhile();  // the copies below wait for the GPU
+  for (size_t i = 0; i < n; ++i) {
+    KL_CUDA_TRY(cudaMemcpyAsync(&gerr[i], ws[i].status, sizeof(int), cudaMemcpyDeviceToHost, st));
     if (!tri[i]) KL_CUDA_TRY(cudaMemcpyAsync(&nsteps[i], ws[i].jst, sizeof(int), cudaMemcpyDeviceToHost, st));
   }
   KL_CUDA_TRY(cudaStreamSynchronize(st));
@@ -1845,9 +1848,10 @@ int gram_factor(const float2* A, int N, int S, double2* G, int* err_dev, cudaStr
 }
 
 int eig_topk_factor(const float2* A, int N, int S, const EigenOptions& opt, double2* U,
-                    double* evals, EigenResult* res, cudaStream_t st) {
+                    double* evals, EigenResult* res, cudaStream_t st, const std::function<void()>& meanwhile) {
   KL_CHECK_ARG(opt.K > 0 && opt.K <= N, "eig_topk_factor: K out of range");
-  if (S <= kGramMaxS && opt.K <= S) return eig_topk_gram({FactorProblem{A, N, S, opt.K, U, evals, res}}, st);
+  if (S <= kGramMaxS && opt.K <= S)
+    return eig_topk_gram({FactorProblem{A, N, S, opt.K, U, evals, res}}, st, meanwhile);
   const int B = block_size(opt, N, S);
   KL_CHECK_ARG(opt.K <= B, "eig_topk_factor: K exceeds the block size");
   double2* Z = nullptr;
@@ -1867,17 +1871,18 @@ int eig_topk_factor(const float2* A, int N, int S, const EigenOptions& opt, doub
   return rc;
 }
 
-int eig_topk_factor_batch(const std::vector<FactorProblem>& pr, const EigenOptions& opt, cudaStream_t st) {
+int eig_topk_factor_batch(const std::vector<FactorProblem>& pr, const EigenOptions& opt, cudaStream_t st,
+                          const std::function<void()>& meanwhile) {
   bool gram = true;
   for (const FactorProblem& f : pr) {
     KL_CHECK_ARG(f.K > 0 && f.K <= f.N, "eig_topk_factor: K out of range");
     gram = gram && f.S <= kGramMaxS && f.K <= f.S;
   }
-  if (gram) return eig_topk_gram(pr, st);
+  if (gram) return eig_topk_gram(pr, st, meanwhile);
   for (const FactorProblem& f : pr) {
     EigenOptions o = opt;
     o.K = f.K;
-    const int rc = eig_topk_factor(f.A, f.N, f.S, o, f.U, f.evals, f.res, st);
+    const int rc = eig_topk_factor(f.A, f.N, f.S, o, f.U, f.evals, f.res, st, nullptr);
     if (rc) return rc;
   }
   return KL_OK;

@@ -191,6 +191,8 @@ size_t spec_part_elems(const SpecGeom& g, int nimg, int nsplit);
 // nk of them from the kernel layout
 size_t spec_kernel_elems(const SpecGeom& g);
 int spec_columns(const SpecGeom& g, const float2* H, int nk, float2* HT, cudaStream_t st);
+// two planes of n floats -> n complex numbers
+int spec_interleave(const float* re, const float* im, size_t n, float2* H, cudaStream_t st);
 // band: nparts partial band spectra [nby][nf] per clip, summed and times scale.
 // H: kernels of all sets in the core's layout, or (natural) the kernel layout.  T
 // receives one spectrum per image.

@@ -364,15 +364,38 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
 }  // namespace
 
 namespace {
-// host kernels -> H (device, kernel layout) -> the spectral core's layout, and the
-// eigenvalues; done on return
-int upload_kernels(kl_socs_plan p, int set, const float2* h, float2* H, const float* scales) {
-  const size_t nb2 = (size_t)p->g.nby * p->g.nbx, k0 = (size_t)set * p->K;
-  KL_CUDA_TRY(cudaMemcpy(H, h, sizeof(float2) * nb2 * p->K, cudaMemcpyHostToDevice));
-  if (int rc = kl::spec_columns(p->sg, H, p->K, p->HT + k0 * kl::spec_kernel_elems(p->sg), nullptr)) return rc;
-  KL_CUDA_TRY(cudaMemcpy(p->lam + k0, scales, sizeof(float) * p->K, cudaMemcpyHostToDevice));
-  KL_CUDA_TRY(cudaStreamSynchronize(nullptr));
-  return KL_OK;
+// kernels of one set from the host, interleaved (im null) or as two planes: copied as
+// they are and put in order on the device -- interleaving 6 MB on the host took
+// longer than the copy.  The kernel layout is kept by adjoint plans, else only on
+// the way to the spectral core's.  Done on return.
+int upload_kernels(kl_socs_plan p, int set, const float* re, const float* im, const float* scales) {
+  const size_t n = (size_t)p->g.nby * p->g.nbx * p->K, k0 = (size_t)set * p->K;
+  void* tmp = nullptr;
+  const size_t tmp_floats = (p->H ? 0 : 2 * n) + (im ? 2 * n : 0);
+  int rc = tmp_floats ? kl::scratch_alloc(&tmp, sizeof(float) * tmp_floats, nullptr, "kernels") : KL_OK;
+  if (rc) return rc;
+  float2* H = p->H ? p->H + set * n : static_cast<float2*>(tmp);
+  float* planes = static_cast<float*>(tmp) + (p->H ? 0 : 2 * n);
+  auto copy = [&](void* dst, const void* src, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) return KL_OK;
+    kl::set_error(std::string("kl_socs_set_kernels: ") + cudaGetErrorString(e));
+    return KL_ERR_CUDA;
+  };
+  if (im) {
+    if (!(rc = copy(planes, re, sizeof(float) * n)) && !(rc = copy(planes + n, im, sizeof(float) * n)))
+      rc = kl::spec_interleave(planes, planes + n, n, H, nullptr);
+  } else {
+    rc = copy(H, re, sizeof(float2) * n);
+  }
+  if (!rc) rc = kl::spec_columns(p->sg, H, p->K, p->HT + k0 * kl::spec_kernel_elems(p->sg), nullptr);
+  if (!rc) rc = copy(p->lam + k0, scales, sizeof(float) * p->K);
+  if (!rc && cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    kl::set_error(std::string("kl_socs_set_kernels: ") + cudaGetErrorString(cudaGetLastError()));
+    rc = KL_ERR_CUDA;
+  }
+  if (tmp) kl::scratch_free(tmp, nullptr);
+  return rc;
 }
 }  // namespace
 
@@ -484,21 +507,13 @@ int kl_socs_set_kernels(kl_socs_plan p, int set, const float* re, const float* i
                         const float* scales) {
   KL_CHECK_ARG(p && re && im && scales, "kl_socs_set_kernels: NULL argument");
   KL_CHECK_ARG(set >= 0 && set < p->nsets, "kl_socs_set_kernels: set out of range");
-  const size_t nb2 = (size_t)p->g.nby * p->g.nbx;
-  std::vector<float2> h(nb2 * p->K);
-  for (size_t i = 0; i < h.size(); ++i) h[i] = make_float2(re[i], im[i]);
-  // in the kernel layout: kept by adjoint plans, else only on the way to the
-  // spectral core's layout
-  float2* H = p->H ? p->H + (size_t)set * p->K * nb2 : nullptr;
-  void* tmp = nullptr;
-  int rc;
-  if (!H) {
-    if ((rc = kl::scratch_alloc(&tmp, sizeof(float2) * h.size(), nullptr, "kernels"))) return rc;
-    H = static_cast<float2*>(tmp);
-  }
-  rc = upload_kernels(p, set, h.data(), H, scales);
-  if (tmp) kl::scratch_free(tmp, nullptr);
-  return rc;
+  return upload_kernels(p, set, re, im, scales);
+}
+
+int kl_socs_set_kernels_c64(kl_socs_plan p, int set, const float* krn, const float* scales) {
+  KL_CHECK_ARG(p && krn && scales, "kl_socs_set_kernels_c64: NULL argument");
+  KL_CHECK_ARG(set >= 0 && set < p->nsets, "kl_socs_set_kernels_c64: set out of range");
+  return upload_kernels(p, set, krn, nullptr, scales);
 }
 
 int kl_socs_set_kernels_device(kl_socs_plan p, int set, const float2* H_dev, const float* lam_dev,

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <functional>
 #include <vector>
 
 namespace kl {
@@ -92,12 +93,13 @@ struct FactorProblem {
 // Top-K eigenpairs of several TCC = A A^H at once (e.g. one per focus value):
 // factors with S <= 256 columns share one batched Gram eigensolve; the rest
 // are solved one after another by subspace iteration.
+// `meanwhile` (may be empty) is host work done once while the GPU solves.
 int eig_topk_factor_batch(const std::vector<FactorProblem>& problems, const EigenOptions& opt,
-                          cudaStream_t st);
+                          cudaStream_t st, const std::function<void()>& meanwhile);
 
 // Operator TCC = A A^H given by its FP32 factor A (N x S).
 int eig_topk_factor(const float2* A, int N, int S, const EigenOptions& opt, double2* U,
-                    double* evals, EigenResult* res, cudaStream_t st);
+                    double* evals, EigenResult* res, cudaStream_t st, const std::function<void()>& meanwhile);
 // Operator given by a materialised FP64 TCC (N x N).
 int eig_topk_dense(const double2* tcc, int N, const EigenOptions& opt, double2* U, double* evals,
                    EigenResult* res, cudaStream_t st);

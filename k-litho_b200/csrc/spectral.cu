@@ -76,7 +76,19 @@ __global__ void k_spec_columns(const float2* __restrict__ H, const SpecGeom g, s
     HT[i] = r < nby ? H[k * nby * g.nbx + (size_t)r * g.nbx + g.Nx + n] : make_float2(0.f, 0.f);
   }
 }
+
+__global__ void k_spec_interleave(const float* __restrict__ re, const float* __restrict__ im, size_t n,
+                                  float2* __restrict__ H) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    H[i] = make_float2(re[i], im[i]);
+}
 }  // namespace
+
+int spec_interleave(const float* re, const float* im, size_t n, float2* H, cudaStream_t st) {
+  k_spec_interleave<<<(int)std::min<size_t>((n + 255) / 256, 148 * 16), 256, 0, st>>>(re, im, n, H);
+  KL_CUDA_TRY(cudaGetLastError());
+  return KL_OK;
+}
 
 int spec_columns(const SpecGeom& g, const float2* H, int nk, float2* HT, cudaStream_t st) {
   const size_t hs = spec::spec_hstride(g), total = hs * nk;

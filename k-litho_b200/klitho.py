@@ -84,6 +84,7 @@ def lib() -> ctypes.CDLL:
         L.kl_resist_contour.argtypes = [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_float,
                                         ctypes.c_float, _vp, _vp, _vp, _vp, _vp]
         L.kl_socs_set_kernels.argtypes = [_vp, ctypes.c_int, _c_float_p, _c_float_p, _c_float_p]
+        L.kl_socs_set_kernels_c64.argtypes = [_vp, ctypes.c_int, _c_float_p, _c_float_p]
         L.kl_socs_forward.argtypes = [_vp, _vp, ctypes.c_int, _vp, _vp]
         L.kl_socs_forward_host.argtypes = [_vp, _c_float_p, ctypes.c_int, _c_float_p, _vp]
         L.kl_mask_spectrum.argtypes = [_vp, _vp, ctypes.c_int, _vp, _vp]
@@ -279,11 +280,9 @@ class SocsPlan:
 
     def set_kernels(self, set_index: int, krn: np.ndarray, scales: np.ndarray) -> None:
         """krn: nk x (2Ny+1)(2Nx+1) complex (kernel-file layout)."""
-        k = np.asarray(krn)
-        re = np.ascontiguousarray(k.real, dtype=np.float32)
-        im = np.ascontiguousarray(k.imag, dtype=np.float32)
+        k = np.ascontiguousarray(krn, dtype=np.complex64)
         sc = np.ascontiguousarray(scales, dtype=np.float32)
-        check(lib().kl_socs_set_kernels(self._h, int(set_index), _fp(re), _fp(im), _fp(sc)),
+        check(lib().kl_socs_set_kernels_c64(self._h, int(set_index), k.ctypes.data_as(_c_float_p), _fp(sc)),
               "kl_socs_set_kernels")
 
     def forward(self, masks_dev, images_dev, nclips: int | None = None, stream=None) -> None:
