@@ -56,9 +56,6 @@ struct SocsGeom {
   int KX;          // rows of the x twiddle table, max(NFM, NBM)
 };
 
-// Largest number of kernel slices the adjoint's spectral stage splits a (clip, set) into.
-constexpr int kSocsMaxSplit = 8;
-
 // Fill geometry; returns KL_OK or KL_ERR_UNSUPPORTED with a message.  With
 // `adjoint`, strips are tall enough (J >= 4Ny+1) to carry the band of the
 // loss gradient dL/dI as well.
@@ -68,9 +65,6 @@ int socs_geometry(int Lx, int Ly, int Nx, int Ny, SocsGeom* g, bool adjoint = fa
 size_t socs_partial_bytes(const SocsGeom& g, int nclips);
 size_t socs_table_x_elems(const SocsGeom& g);  // float2 elements of tx
 size_t socs_table_y_elems(const SocsGeom& g);  // float2 elements of ty
-// kernel slices per (clip, set) of the adjoint's spectral launch of `nclips` clips
-int socs_choose_split(const SocsGeom& g, int nclips, int nsets, int K);
-
 // Plan-time twiddle tables (stream-ordered).
 int socs_build_tables(const SocsGeom& g, float2* tx, float2* ty, cudaStream_t st);
 
@@ -143,7 +137,7 @@ size_t gen_rowbins_bytes(const GenGeom& g, int nrows_img, int nbins);  // R / Q 
 size_t gen_band_bytes(const GenGeom& g, int n, int nparts, int nrows, int ncols);
 size_t gen_table_elems(const GenGeom& g);  // twb + twl + tw2 + rootLy (float2)
 int gen_build_tables(const GenGeom& g, float2* tables, cudaStream_t st);
-// kernel slices per image of the adjoint's spectral launch
+// kernel slices per image of the adjoint's spectral launch on grids above 128 points
 int gen_choose_split(const GenGeom& g, int nimg, int K);
 int gen_choose_parts(const GenGeom& g, int n, int ncols);
 
@@ -165,7 +159,6 @@ int gen_launch_rowvjp(const GenGeom& g, const float2* tables, float2* Q, int nim
 int gen_launch_vjp_spectral(const GenGeom& g, const float2* band, int nparts, const float2* gband, int gparts,
                             int nclips, const float2* H, const float* lam, int K, int nsets, int nsplit, float2* gam,
                             cudaStream_t st);
-int gen_launch_gradT(const GenGeom& g, const float2* gam, int nclips, int nparts, float2* Tg, cudaStream_t st);
 int gen_launch_vjp_source(const GenGeom& g, const float2* band, int nparts, const float2* gband, int gparts,
                           int nimg, int nsets, const float2* Hs, int S, const float* Jw, const int* src_id,
                           int nsplit, float* grad_src, cudaStream_t st);
@@ -200,6 +193,22 @@ int spec_interleave(const float* re, const float* im, size_t n, float2* H, cudaS
 int spec_launch(const SpecGeom& g, const float2* band, int nparts, float scale, int nimg, const float2* H, bool natural,
                 const float* lam, int K, int nsets, int nsplit, float2* part, float2* T,
                 unsigned* done, cudaStream_t st);
+
+// The adjoint's spectral core (adjoint_spectral.cu), grids up to 128 points: Gam of
+// each image in nsplit * adjoint_shares shares [nby][nbx].  gband: gparts partial
+// spectra of dL/dI [4Ny+1][2Nx+1] per image; H in the core's layout; gamma: scratch.
+constexpr int kAdjointMaxSplit = 32;
+bool adjoint_core(const SpecGeom& g);
+int adjoint_shares(const SpecGeom& g);
+size_t adjoint_gamma_elems(const SpecGeom& g, int nimg);
+int adjoint_choose_split(const SpecGeom& g, int nimg, int K);
+int adjoint_launch(const SpecGeom& g, const float2* band, int nparts, float scale, const float2* gband, int gparts,
+                   int nimg, const float2* H, const float* lam, int K, int nsets, int nsplit, float* gamma, float2* gam,
+                   cudaStream_t st);
+// the shares of Gam of each clip (nparts of them) -> half-plane spectrum of dL/dm, T(a, b)
+// at strides sa, sb for |a| <= ay, 0 <= b < nb (zero outside the band)
+int adjoint_gradient(const SpecGeom& g, const float2* gam, int nclips, int nparts, int ay, int nb, int sa, int sb, float2* T,
+                     cudaStream_t st);
 
 }  // namespace kl
 

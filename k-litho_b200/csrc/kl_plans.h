@@ -14,7 +14,7 @@ struct kl_socs_plan_s {
   int device = 0;
   bool adjoint = false;
   void* buffers = nullptr;   // the allocation that the device pointers below lie in
-  float2* H = nullptr;       // nsets x K x nby x nbx (adjoint plans)
+  float2* H = nullptr;       // nsets x K x nby x nbx (adjoint plans with grids above 128 points)
   float2* HT = nullptr;      // the same in the spectral core's layout
   unsigned* done = nullptr;  // slice counters of the spectral core
   kl::SpecGeom sg{};
@@ -32,7 +32,8 @@ struct kl_socs_plan_s {
   cudaEvent_t hev[3] = {nullptr, nullptr, nullptr};
   // adjoint state (kl_socs_plan_create_adjoint)
   float2* gpart = nullptr;   // strip partials of the spectrum of dL/dI
-  float2* gam = nullptr;     // per-slice Gam partials
+  float* gamma = nullptr;    // dL/dI on the spectral grid
+  float2* gam = nullptr;     // shares of Gam
   float2* Tg = nullptr;      // half-plane spectrum of dL/dm
   int last_vjp_clips = 0;
   // optional stage timing: 4 events per kl_socs_forward
@@ -99,11 +100,6 @@ size_t vjp_gpart_bytes(const SocsGeom& g, int nimg);
 int vjp_launch_inverse(const SocsGeom& g, const float2* tx, const float2* ty, const float2* T,
                        int nclips, int nsets, const float* targets, float alpha,
                        float thr, float* images, double* loss, float2* gpart, cudaStream_t st);
-int vjp_launch_spectral(const SocsGeom& g, const float2* partial, const float2* gpart, int nclips,
-                        const float2* H, const float* lam, int K, int nsets, int nsplit,
-                        float2* gam_out, cudaStream_t st);
-int vjp_launch_gradT(const SocsGeom& g, const float2* gam, int nclips, int nparts, float2* T,
-                     cudaStream_t st);
 int vjp_launch_source(const SocsGeom& g, const float2* partial, const float2* gpart, int nimg,
                       int nsets, const float2* Hs, const float* Jw, const int* src_id, int S,
                       int nsplit, float* grad_src, cudaStream_t st);

@@ -148,8 +148,8 @@ int spectral(kl_socs_plan p, int nclips, int nsplit, cudaStream_t st) {
                          false, p->lam, p->K, p->nsets, nsplit, p->part, p->T, p->done, st);
 }
 
-// buffers of the spectral core: the kernels in its layout (and, for the adjoint,
-// the kernel layout), spectra for any batch up to max_clips, slice counters
+// buffers of the spectral core: the kernels in its layout (and, for the adjoint on
+// grids above 128 points, the kernel layout), spectra for any batch up to max_clips, slice counters
 void spectral_pieces(kl_socs_plan p, Pieces& mem) {
   const kl::SpecGeom& g = p->sg;
   const size_t nk = (size_t)p->K * p->nsets, nimg = (size_t)p->max_clips * p->nsets;
@@ -157,11 +157,28 @@ void spectral_pieces(kl_socs_plan p, Pieces& mem) {
     p->part_cap = std::max(p->part_cap, kl::spec_part_elems(g, n * p->nsets,
                                                             kl::spec_choose_split(g, n * p->nsets, p->K)));
   mem.add(&p->HT, sizeof(float2) * nk * kl::spec_kernel_elems(g));
-  if (p->adjoint) mem.add(&p->H, sizeof(float2) * nk * g.nby * g.nbx);
+  if (p->adjoint && !kl::adjoint_core(g)) mem.add(&p->H, sizeof(float2) * nk * g.nby * g.nbx);
   mem.add(&p->lam, sizeof(float) * nk);
   mem.add(&p->T, sizeof(float2) * nimg * g.nty * g.ntx);
   mem.add(&p->part, sizeof(float2) * p->part_cap);
   mem.add(&p->done, sizeof(unsigned) * nimg);
+}
+
+// kernel slices of the adjoint's spectral stage, and its shares of Gam per image
+int adjoint_split(kl_socs_plan p, int nimg) {
+  return kl::adjoint_core(p->sg) ? kl::adjoint_choose_split(p->sg, nimg, p->K) : kl::gen_choose_split(p->gg, nimg, p->K);
+}
+int adjoint_parts(kl_socs_plan p, int nsplit) {
+  return kl::adjoint_core(p->sg) ? nsplit * kl::adjoint_shares(p->sg) : nsplit;
+}
+// the largest number of shares any batch size needs
+size_t adjoint_shares_cap(kl_socs_plan p) {
+  size_t cap = 0;
+  for (int n = 1; n <= p->max_clips; ++n) {
+    const int nimg = n * p->nsets;
+    cap = std::max(cap, (size_t)nimg * adjoint_parts(p, adjoint_split(p, nimg)));
+  }
+  return cap;
 }
 
 // a new plan's kernels are zero, as are its counters; the default stream's work
@@ -248,14 +265,12 @@ int create_gen_plan(kl_socs_plan* plan, int Lx, int Ly, int Nx, int Ny, int nk, 
   mem.add(&p->band, kl::gen_band_bytes(gg, max_clips, pmax, gg.nby, gg.nf));
   mem.add(&p->Q, kl::gen_rowbins_bytes(gg, max_clips * nsets, gg.ntx));
   if (adjoint) {
-    int gmax = 0, slices = 0;
-    for (int n = 1; n <= max_clips; ++n) {
-      gmax = std::max(gmax, kl::gen_choose_parts(gg, n * nsets, gg.ntx));
-      slices = std::max(slices, n * nsets * kl::gen_choose_split(gg, n * nsets, nk));
-    }
+    int gmax = 0;
+    for (int n = 1; n <= max_clips; ++n) gmax = std::max(gmax, kl::gen_choose_parts(gg, n * nsets, gg.ntx));
     p->gparts_max = gmax;
     mem.add(&p->gband, kl::gen_band_bytes(gg, max_clips * nsets, gmax, gg.nty, gg.ntx));
-    mem.add(&p->gam, sizeof(float2) * gg.nby * gg.nbx * slices);
+    mem.add(&p->gamma, sizeof(float) * kl::adjoint_gamma_elems(p->sg, max_clips * nsets));
+    mem.add(&p->gam, sizeof(float2) * gg.nby * gg.nbx * adjoint_shares_cap(p));
     mem.add(&p->Tg, sizeof(float2) * (size_t)max_clips * gg.nf * gg.nby);
   }
   if ((rc = mem.allocate(&p->buffers)) || (rc = kl::gen_build_tables(gg, p->gtab, nullptr)) || (rc = finish_plan(p))) {
@@ -309,10 +324,9 @@ int create_plan(kl_socs_plan* plan, int Lx, int Ly, int Nx, int Ny, int nk, int 
     }
   }
   if (adjoint) {
-    int slices = 0;  // the largest clips x slices product any batch size needs
-    for (int n = 1; n <= max_clips; ++n) slices = std::max(slices, n * kl::socs_choose_split(g, n, nsets, nk));
     mem.add(&p->gpart, kl::vjp_gpart_bytes(g, max_clips * nsets));
-    mem.add(&p->gam, sizeof(float2) * g.nby * g.nbx * slices * nsets);
+    mem.add(&p->gamma, sizeof(float) * kl::adjoint_gamma_elems(p->sg, max_clips * nsets));
+    mem.add(&p->gam, sizeof(float2) * g.nby * g.nbx * adjoint_shares_cap(p));
     mem.add(&p->Tg, sizeof(float2) * (size_t)max_clips * g.nty * g.ntx);
   }
   if ((rc = mem.allocate(&p->buffers)) || (rc = kl::socs_build_tables(g, p->tx, p->ty, nullptr)) ||
@@ -334,7 +348,7 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
   const kl::GenGeom& g = p->gg;
   const int nimg = nclips * p->nsets;
   const int ns = kl::spec_choose_split(p->sg, nimg, p->K);
-  const int ns_adj = kl::gen_choose_split(g, nimg, p->K);
+  const int ns_adj = adjoint_split(p, nimg);
   const int nparts = kl::gen_choose_parts(g, nclips, g.nf);
   const int gparts = kl::gen_choose_parts(g, nimg, g.ntx);
   int rc;
@@ -350,10 +364,15 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
   if ((rc = kl::gen_launch_rowvjp(g, p->gtab, p->Q, nimg, p->nsets, targets, alpha, threshold, images, loss, st)))
     return rc;
   if ((rc = kl::gen_launch_colfwd(g, p->gtab, p->Q, nimg, g.ntx, 2 * g.Ny, 1.0f, gparts, p->gband, st))) return rc;
-  if ((rc = kl::gen_launch_vjp_spectral(g, p->band, nparts, p->gband, gparts, nclips, p->H, p->lam, p->K, p->nsets,
-                                        ns_adj, p->gam, st)))
+  rc = kl::adjoint_core(p->sg)
+           ? kl::adjoint_launch(p->sg, p->band, nparts, 1.0f, p->gband, gparts, nimg, p->HT, p->lam, p->K, p->nsets, ns_adj,
+                                p->gamma, p->gam, st)
+           : kl::gen_launch_vjp_spectral(g, p->band, nparts, p->gband, gparts, nclips, p->H, p->lam, p->K, p->nsets,
+                                         ns_adj, p->gam, st);
+  if (rc) return rc;
+  if ((rc = kl::adjoint_gradient(p->sg, p->gam, nclips, p->nsets * adjoint_parts(p, ns_adj), g.Ny, g.nf, 1, g.nby, p->Tg,
+                                 st)))
     return rc;
-  if ((rc = kl::gen_launch_gradT(g, p->gam, nclips, p->nsets * ns_adj, p->Tg, st))) return rc;
   if ((rc = kl::gen_launch_colinv(g, p->gtab, p->Tg, nclips, g.Ny, g.nf, p->Q, st))) return rc;
   if ((rc = kl::gen_launch_rowinv(g, p->gtab, p->Q, nclips, g.nf, grad, st))) return rc;
   p->last_vjp_clips = nclips;
@@ -366,8 +385,8 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
 namespace {
 // kernels of one set from the host, interleaved (im null) or as two planes: copied as
 // they are and put in order on the device -- interleaving 6 MB on the host took
-// longer than the copy.  The kernel layout is kept by adjoint plans, else only on
-// the way to the spectral core's.  Done on return.
+// longer than the copy.  The kernel layout is kept where an adjoint needs it,
+// else only on the way to the spectral core's.  Done on return.
 int upload_kernels(kl_socs_plan p, int set, const float* re, const float* im, const float* scales) {
   const size_t n = (size_t)p->g.nby * p->g.nbx * p->K, k0 = (size_t)set * p->K;
   void* tmp = nullptr;
@@ -452,11 +471,13 @@ int kl_socs_vjp(kl_socs_plan p, const float* masks, const float* targets, int nc
            : kl::vjp_launch_inverse(g, p->tx, p->ty, p->T, nclips, p->nsets, targets, alpha, threshold, images,
                                     loss, p->gpart, st);
   if (rc) return rc;
-  const int ns2 = kl::socs_choose_split(g, nclips, p->nsets, p->K);
-  if ((rc = kl::vjp_launch_spectral(g, p->partial, p->gpart, nclips, p->H, p->lam, p->K, p->nsets,
-                                    ns2, p->gam, st)))
+  const int ns2 = adjoint_split(p, nclips * p->nsets);
+  if ((rc = kl::adjoint_launch(p->sg, p->partial, g.nS, 1.0f / ((float)g.Lx * (float)g.Ly), p->gpart, g.nS,
+                               nclips * p->nsets, p->HT, p->lam, p->K, p->nsets, ns2, p->gamma, p->gam, st)))
     return rc;
-  if ((rc = kl::vjp_launch_gradT(g, p->gam, nclips, p->nsets * ns2, p->Tg, st))) return rc;
+  if ((rc = kl::adjoint_gradient(p->sg, p->gam, nclips, p->nsets * adjoint_parts(p, ns2), 2 * g.Ny, g.ntx, g.ntx, 1, p->Tg,
+                                 st)))
+    return rc;
   // the gradient is a band-limited synthesis like the image: on the tensor
   // cores unless the plan asks for the CUDA-core engine
   const bool tcg = p->bhi && p->synth != KL_SYNTH_CUDA_CORES && kl::synth_tc_aligned(grad);

@@ -118,15 +118,6 @@ size_t socs_partial_bytes(const SocsGeom& g, int nclips) {
 size_t socs_table_x_elems(const SocsGeom& g) { return (size_t)g.KX * g.V; }
 size_t socs_table_y_elems(const SocsGeom& g) { return (size_t)g.nS * g.nty; }
 
-int socs_choose_split(const SocsGeom& g, int nclips, int nsets, int K) {
-  // enough CTAs to cover the GPU about twice; slices of at least 3 kernels
-  const int ctas = nclips * nsets;
-  int ns = 1;
-  while (ns < kSocsMaxSplit && ctas * ns < 2 * 148 && K / (2 * ns) >= 3) ns *= 2;
-  (void)g;
-  return ns;
-}
-
 // ---------------------------------------------------------------------------
 // plan-time tables: tx[k][l'] = e^{-2 pi i k l'/Lx}, ty[s][a+2Ny] = e^{+2 pi i a s/Ly}
 // ---------------------------------------------------------------------------

@@ -139,9 +139,15 @@ int gen_choose_split(const GenGeom& g, int nimg, int K) {
 }
 
 int gen_choose_parts(const GenGeom& g, int n, int ncols) {
-  // enough CTAs of the column transform to cover the GPU, at least 4 strips each
-  const int groups = (ncols + kW - 1) / kW;
+  // enough CTAs of the column transform to cover the GPU, at least 4 strips each; of
+  // the blocked one once, at least 2 blocks of rows each
   int np = 1;
+  if (!g.ystrip) {
+    const int cols = (ncols + 15) / 16;
+    while (cols * n * np < kSMs && g.nS / (2 * np) >= 2) np *= 2;
+    return np;
+  }
+  const int groups = (ncols + kW - 1) / kW;
   while (groups * n * np < 2 * kSMs && g.nS / (2 * np) >= 4) np *= 2;
   return np;
 }
@@ -272,7 +278,8 @@ __global__ void __launch_bounds__(kT) k_gen_rowfwd(const float* __restrict__ src
 }
 
 // ---------------------------------------------------------------------------
-// 2. col_fwd: R[n][y][fx] -> band[n][part][fy + Yb][fx], |fy| <= Yb, times scale
+// 2. col_fwd: R[n][y][fx] -> band[n][part][fy + Yb][fx], |fy| <= Yb, times scale;
+// periods of strips (Ly a multiple of 32)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R, int ncols, int Yb,
                                                    const GenGeom g, const float2* __restrict__ rly,
@@ -290,66 +297,113 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R,
   float2 acc[MT];
 #pragma unroll
   for (int t = 0; t < MT; ++t) acc[t] = make_float2(0.f, 0.f);
-  if (g.ystrip) {
-    const int nS = g.nS;
-    const int s0 = (int)((long long)nS * part / nparts), s1 = (int)((long long)nS * (part + 1) / nparts);
-    WarpFFT<1, -1> wf;
-    wf.init(lane);
-    const int q = brev5(lane);
-    const int fy0 = q - 32 * ((q + Yb) / 32);  // smallest fy >= -Yb with fy = q (mod 32)
-    // the next strip's row bin and phases are loaded while this strip is transformed
-    float2 rn = make_float2(0.f, 0.f), pn[MT];
-    auto fetch = [&](int s) {
-      rn = __ldg(Rn + (size_t)(s + nS * lane) * ncols + fx);
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const int fy = fy0 + 32 * t;
-        pn[t] = fy <= Yb ? __ldg(rly + mod_pos(fy * s, Ly)) : make_float2(1.f, 0.f);
-      }
-    };
-    if (s0 < s1) fetch(s0);
-    for (int s = s0; s < s1; ++s) {
-      float2 v[1] = {rn};
-      float2 p[MT];
-#pragma unroll
-      for (int t = 0; t < MT; ++t) p[t] = pn[t];
-      if (s + 1 < s1) fetch(s + 1);
-      wf.run(v, lane);
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const int fy = fy0 + 32 * t;
-        if (fy <= Yb) acc[t] = cfma(v[0], cconj(p[t]), acc[t]);
-      }
-    }
+  const int nS = g.nS;
+  const int s0 = (int)((long long)nS * part / nparts), s1 = (int)((long long)nS * (part + 1) / nparts);
+  WarpFFT<1, -1> wf;
+  wf.init(lane);
+  const int q = brev5(lane);
+  const int fy0 = q - 32 * ((q + Yb) / 32);  // smallest fy >= -Yb with fy = q (mod 32)
+  // the next strip's row bin and phases are loaded while this strip is transformed
+  float2 rn = make_float2(0.f, 0.f), pn[MT];
+  auto fetch = [&](int s) {
+    rn = __ldg(Rn + (size_t)(s + nS * lane) * ncols + fx);
 #pragma unroll
     for (int t = 0; t < MT; ++t) {
       const int fy = fy0 + 32 * t;
-      if (fy <= Yb) out[(size_t)(fy + Yb) * ncols + fx] = cscale(acc[t], scale);
+      pn[t] = fy <= Yb ? __ldg(rly + mod_pos(fy * s, Ly)) : make_float2(1.f, 0.f);
     }
-  } else {
-    const int y0 = (int)((long long)Ly * part / nparts), y1 = (int)((long long)Ly * (part + 1) / nparts);
-    int m[MT];
+  };
+  if (s0 < s1) fetch(s0);
+  for (int s = s0; s < s1; ++s) {
+    float2 v[1] = {rn};
+    float2 p[MT];
 #pragma unroll
-    for (int t = 0; t < MT; ++t) m[t] = mod_pos((-Yb + lane + 32 * t) * y0, Ly);
-    for (int y = y0; y < y1; ++y) {
-      const float2 v = __ldg(Rn + (size_t)y * ncols + fx);
+    for (int t = 0; t < MT; ++t) p[t] = pn[t];
+    if (s + 1 < s1) fetch(s + 1);
+    wf.run(v, lane);
 #pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const int fy = -Yb + lane + 32 * t;
-        if (fy <= Yb) {
-          acc[t] = cfma(v, cconj(__ldg(rly + m[t])), acc[t]);
-          m[t] += fy;
-          if (m[t] >= Ly) m[t] -= Ly;
-          else if (m[t] < 0) m[t] += Ly;
-        }
+    for (int t = 0; t < MT; ++t) {
+      const int fy = fy0 + 32 * t;
+      if (fy <= Yb) acc[t] = cfma(v[0], cconj(p[t]), acc[t]);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < MT; ++t) {
+    const int fy = fy0 + 32 * t;
+    if (fy <= Yb) out[(size_t)(fy + Yb) * ncols + fx] = cscale(acc[t], scale);
+  }
+}
+
+// The same for Ly not a multiple of 32: the DFT over y as small matrix products, 32
+// rows at a time.  y = 32 s + j: a CTA multiplies the block's rows by e^{-2 pi i fy j/Ly}
+// (the same 32 x 64 table for every block) and turns the block's sum by
+// e^{-2 pi i fy 32 s/Ly}.  Thread = one column fx, four fy.  One frequency per lane with
+// both factors gathered for every row took 102 us for seven 1000 x 744 clips.
+__global__ void __launch_bounds__(kT) k_gen_colfwd_blocks(const float2* __restrict__ R, int ncols, int Yb,
+                                                          const GenGeom g, const float2* __restrict__ rly, int nparts,
+                                                          float scale, float2* __restrict__ band) {
+  __shared__ float2 Rt[32][16];
+  __shared__ float2 Wt[32][64];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int nyo = 2 * Yb + 1, Ly = g.Ly;
+  const int fx0 = blockIdx.x * 16, r0 = blockIdx.y * 64;  // rows r = fy + Yb of the band
+  const int n = blockIdx.z / nparts, part = blockIdx.z - n * nparts;
+  const int s0 = (int)((long long)g.nS * part / nparts), s1 = (int)((long long)g.nS * (part + 1) / nparts);
+  const int nr = min(64, nyo - r0), nq = (nr + 15) / 16;
+  for (int i = tid; i < 32 * 64; i += kT) {
+    const int j = i >> 6, fy = r0 + (i & 63) - Yb;
+    Wt[j][i & 63] = cconj(__ldg(rly + mod_pos(fy * j, Ly)));
+  }
+  dep_wait();
+  dep_launch();
+  const float2* Rn = R + (size_t)n * Ly * ncols + fx0 + tx;
+  const bool colok = fx0 + tx < ncols;
+  float2 next[2];
+  auto fetch = [&](int s) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int y = 32 * s + ty + 16 * h;
+      next[h] = colok && y < Ly ? __ldg(Rn + (size_t)y * ncols) : make_float2(0.f, 0.f);
+    }
+  };
+  float2 acc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) acc[q] = make_float2(0.f, 0.f);
+  if (s0 < s1) fetch(s0);
+  for (int s = s0; s < s1; ++s) {
+    Rt[ty][tx] = next[0];
+    Rt[ty + 16][tx] = next[1];
+    __syncthreads();
+    if (s + 1 < s1) fetch(s + 1);
+    float2 rot[4], blk[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      rot[q] = cconj(__ldg(rly + mod_pos((r0 + ty + 16 * q - Yb) * (32 * s), Ly)));
+      blk[q] = make_float2(0.f, 0.f);
+    }
+    if (nq > 2) {
+#pragma unroll 8
+      for (int j = 0; j < 32; ++j) {
+        const float2 r = Rt[j][tx];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) blk[q] = cfma(r, Wt[j][ty + 16 * q], blk[q]);
+      }
+    } else {
+#pragma unroll 8
+      for (int j = 0; j < 32; ++j) {
+        const float2 r = Rt[j][tx];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) blk[q] = cfma(r, Wt[j][ty + 16 * q], blk[q]);
       }
     }
 #pragma unroll
-    for (int t = 0; t < MT; ++t) {
-      const int fy = -Yb + lane + 32 * t;
-      if (fy <= Yb) out[(size_t)(fy + Yb) * ncols + fx] = cscale(acc[t], scale);
-    }
+    for (int q = 0; q < 4; ++q) acc[q] = cfma(blk[q], rot[q], acc[q]);
+    __syncthreads();
   }
+  float2* out = band + ((size_t)n * nparts + part) * nyo * ncols + fx0 + tx;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    if (colok && ty + 16 * q < nr) out[(size_t)(r0 + ty + 16 * q) * ncols] = cscale(acc[q], scale);
 }
 
 // ---------------------------------------------------------------------------
@@ -374,53 +428,98 @@ __global__ void __launch_bounds__(kT) k_gen_colinv(const float2* __restrict__ T,
   dep_wait();
   dep_launch();
   for (int s = s0; s < s1; ++s) {
-    int nr = 32;
-    if (g.ystrip) {
-      for (int i = threadIdx.x; i < lda; i += kT) ph[i] = __ldg(rly + mod_pos((i - A) * s, Ly));
-      __syncthreads();
-      const int a0 = lane - 32 * ((lane + A) / 32);  // smallest a >= -A with a = lane (mod 32)
-      for (int b = warp; b < nbins; b += kW) {
-        // the column's terms a = a0 + 32 t (at most 8: 2A + 1 <= 255), loads issued together
-        float2 tv[8];
-        const float2* tp = Ti + (size_t)b * lda + A;
+    for (int i = threadIdx.x; i < lda; i += kT) ph[i] = __ldg(rly + mod_pos((i - A) * s, Ly));
+    __syncthreads();
+    const int a0 = lane - 32 * ((lane + A) / 32);  // smallest a >= -A with a = lane (mod 32)
+    for (int b = warp; b < nbins; b += kW) {
+      // the column's terms a = a0 + 32 t (at most 8: 2A + 1 <= 255), loads issued together
+      float2 tv[8];
+      const float2* tp = Ti + (size_t)b * lda + A;
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const int a = a0 + 32 * t;
-          tv[t] = a <= A ? __ldg(tp + a) : make_float2(0.f, 0.f);
-        }
-        float2 f = make_float2(0.f, 0.f);
+      for (int t = 0; t < 8; ++t) {
+        const int a = a0 + 32 * t;
+        tv[t] = a <= A ? __ldg(tp + a) : make_float2(0.f, 0.f);
+      }
+      float2 f = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const int a = a0 + 32 * t;
-          if (a <= A) f = cfma(tv[t], ph[a + A], f);
-        }
-        float2 v[1] = {f};
-        wf.run(v, lane);
-        Qs[br * qp + b] = cscale(v[0], b == 0 ? 1.f : 2.f);
+      for (int t = 0; t < 8; ++t) {
+        const int a = a0 + 32 * t;
+        if (a <= A) f = cfma(tv[t], ph[a + A], f);
       }
-    } else {
-      const int y = s * 32 + lane;
-      nr = min(32, Ly - s * 32);
-      for (int b = warp; b < nbins; b += kW) {
-        float2 f = make_float2(0.f, 0.f);
-        if (y < Ly) {
-          int m = mod_pos(-A * y, Ly);
-          const float2* tp = Ti + (size_t)b * lda;
-          for (int a = 0; a < lda; ++a) {
-            f = cfma(__ldg(tp + a), __ldg(rly + m), f);
-            m += y;
-            if (m >= Ly) m -= Ly;
-          }
-        }
-        Qs[lane * qp + b] = cscale(f, b == 0 ? 1.f : 2.f);
-      }
+      float2 v[1] = {f};
+      wf.run(v, lane);
+      Qs[br * qp + b] = cscale(v[0], b == 0 ? 1.f : 2.f);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nr * nbins; i += kT) {
+    for (int i = threadIdx.x; i < 32 * nbins; i += kT) {
       const int j = i / nbins, b = i - j * nbins;
-      const int y = g.ystrip ? s + g.nS * j : s * 32 + j;
-      Qi[(size_t)y * nbins + b] = Qs[j * qp + b];
+      Qi[(size_t)(s + g.nS * j) * nbins + b] = Qs[j * qp + b];
     }
+    __syncthreads();
+  }
+}
+
+// The same for Ly not a multiple of 32, by blocks of 32 rows y = 32 s + j: T is turned
+// by e^{2 pi i a 32 s/Ly} on its way to shared memory, 32 terms a at a time, and
+// multiplied by the 32 x 32 table e^{2 pi i a j/Ly}.  Thread = row j, every eighth bin
+// (MB of them) of SB blocks: one table value serves all.  A row per lane with both
+// factors gathered for every term took 20 us for 14 images of 1000 x 744.
+template <int MB, int SB>
+__global__ void __launch_bounds__(kT) k_gen_colinv_blocks(const float2* __restrict__ T, int A, int nbins,
+                                                          const GenGeom g, const float2* __restrict__ rly,
+                                                          float2* __restrict__ Q) {
+  extern __shared__ float4 smem4[];
+  float2* Wt = reinterpret_cast<float2*>(smem4);  // [32 a][32 j]
+  float2* Tt = Wt + 32 * 32;                      // [SB][32 a][8 MB]; at the end [32 j][nbins]
+  constexpr int NB = kW * MB;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lda = 2 * A + 1, Ly = g.Ly, s0 = blockIdx.x * SB, img = blockIdx.y;
+  const float2* Ti = T + (size_t)img * nbins * lda;
+  float2 acc[SB][MB];
+#pragma unroll
+  for (int s = 0; s < SB; ++s)
+#pragma unroll
+    for (int q = 0; q < MB; ++q) acc[s][q] = make_float2(0.f, 0.f);
+  float2 ph[SB];  // e^{2 pi i a 32 s/Ly} of this lane's a
+#pragma unroll
+  for (int s = 0; s < SB; ++s) ph[s] = __ldg(rly + mod_pos((lane - A) * (32 * (s0 + s)), Ly));
+  dep_wait();
+  dep_launch();
+  for (int a0 = 0; a0 < lda; a0 += 32) {
+#pragma unroll
+    for (int i = threadIdx.x; i < 32 * 32; i += kT) Wt[i] = __ldg(rly + mod_pos((a0 + (i >> 5) - A) * (i & 31), Ly));
+    const int a = a0 + lane;
+#pragma unroll
+    for (int q = 0; q < MB; ++q) {
+      const int b = warp + kW * q;
+      const float2 t = a < lda && b < nbins ? __ldg(Ti + (size_t)b * lda + a) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int s = 0; s < SB; ++s) Tt[(size_t)(s * 32 + lane) * NB + b] = cmul(t, ph[s]);
+    }
+#pragma unroll
+    for (int s = 0; s < SB; ++s) ph[s] = __ldg(rly + mod_pos((a + 32 - A) * (32 * (s0 + s)), Ly));
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+      const float2 w = Wt[k * 32 + lane];
+#pragma unroll
+      for (int s = 0; s < SB; ++s)
+#pragma unroll
+        for (int q = 0; q < MB; ++q) acc[s][q] = cfma(Tt[(size_t)(s * 32 + k) * NB + warp + kW * q], w, acc[s][q]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int s = 0; s < SB; ++s) {
+#pragma unroll
+    for (int q = 0; q < MB; ++q) {
+      const int b = warp + kW * q;
+      if (b < nbins) Tt[lane * nbins + b] = cscale(acc[s][q], b == 0 ? 1.f : 2.f);
+    }
+    __syncthreads();
+    const int y0 = 32 * (s0 + s), n = min(32, Ly - y0) * nbins;
+    float2* Qi = Q + ((size_t)img * Ly + y0) * nbins;
+    for (int i = threadIdx.x; i < n; i += kT) Qi[i] = Tt[i];
     __syncthreads();
   }
 }
@@ -573,6 +672,11 @@ int gen_launch_colfwd(const GenGeom& g, const float2* tables, const float2* R, i
     set_error("gen_launch_colfwd: band taller than 256 rows");
     return KL_ERR_UNSUPPORTED;
   }
+  if (!g.ystrip) {
+    KL_CUDA_TRY(launch_dependent(k_gen_colfwd_blocks, dim3((ncols + 15) / 16, (2 * Yb + 64) / 64, n * nparts), kT, 0, st, R,
+                                 ncols, Yb, g, tables + off_rly(g), nparts, scale, band));
+    return KL_OK;
+  }
   dim3 grid((ncols + kW - 1) / kW, n, nparts);
   KL_CUDA_TRY(launch_dependent(k_gen_colfwd, grid, kT, 0, st, R, ncols, Yb, g, tables + off_rly(g), scale, band));
   return KL_OK;
@@ -581,6 +685,19 @@ int gen_launch_colfwd(const GenGeom& g, const float2* tables, const float2* R, i
 int gen_launch_colinv(const GenGeom& g, const float2* tables, const float2* T, int nimg, int A,
                       int nbins, float2* Q, cudaStream_t st) {
   if (nimg <= 0) return KL_OK;
+  if (!g.ystrip) {
+    auto launch = [&](auto kern, int mb, int sb) -> int {
+      const size_t sm = sizeof(float2) * (size_t)(32 * 32 + sb * 32 * kW * mb);
+      if (int rc = set_smem(kern, sm)) return rc;
+      KL_CUDA_TRY(launch_dependent(kern, dim3((g.nS + sb - 1) / sb, nimg), kT, sm, st, T, A, nbins, g,
+                                   tables + off_rly(g), Q));
+      return KL_OK;
+    };
+    // bins per thread by the band; several blocks per CTA where that leaves registers
+    if (nbins <= 32) return launch(k_gen_colinv_blocks<4, 4>, 4, 4);
+    if (nbins <= 64) return launch(k_gen_colinv_blocks<8, 2>, 8, 2);
+    return launch(k_gen_colinv_blocks<16, 1>, 16, 1);
+  }
   // a few strips per CTA so the image's T is reused from L1, enough CTAs to fill the GPU
   int spc = 1;
   while (spc < 8 && (long long)nimg * ((g.nS + 2 * spc - 1) / (2 * spc)) >= 4 * kSMs) spc *= 2;

@@ -13,13 +13,14 @@
 //   row_vjp       image rows from Q (as row_inv), resist, loss, dL/dI, and the
 //                 row DFT of dL/dI for gx in [0, 2Nx], written over Q in place
 //   col_fwd       (socs_gen.cu) those rows' DFT along y, |gy| <= 2Ny
-//   vjp_spectral  per (image, kernel slice) a cluster of G/32 CTAs, each owning
+//   vjp_spectral  (adjoint_spectral.cu up to 128 grid points; here above)
+//                 per (image, kernel slice) a cluster of G/32 CTAs, each owning
 //                 the grid columns x = c + (G/32) j: gam at its columns, the
 //                 fields recomputed, w = conj(e) gam transformed back (y by the
 //                 transposed warp FFT from registers, x by a 32-point FFT) and
 //                 accumulated against H_k; the CTAs sum Gam through
 //                 distributed shared memory
-//   gradT         Gam -> half-plane spectrum of dL/dm
+//   gradT         (adjoint_spectral.cu) Gam -> half-plane spectrum of dL/dm
 //   col_inv, row_inv (socs_gen.cu) the gradient image
 //   vjp_source    dL/dJ through the TCC factor A (one pass per source point)
 #include <cooperative_groups.h>
@@ -430,29 +431,6 @@ __global__ void __launch_bounds__(kT, 1) k_gen_vjp_spectral(const float2* __rest
 }
 
 // ---------------------------------------------------------------------------
-// gradT: Tg[clip][b][a + Ny] = sum_parts (conj Gam[a][b] + Gam[-a][-b]) / (Lx Ly),
-// |a| <= Ny, b in [0, Nx] (the layout col_inv reads)
-// ---------------------------------------------------------------------------
-__global__ void k_gen_gradT(const float2* __restrict__ gam, const GenGeom g, int nparts, float2* __restrict__ Tg) {
-  const int clip = blockIdx.x;
-  const size_t nb2 = (size_t)g.nby * g.nbx;
-  const float2* p0 = gam + (size_t)clip * nparts * nb2;
-  const float s = 1.0f / ((float)g.Lx * (float)g.Ly);
-  float2* To = Tg + (size_t)clip * g.nf * g.nby;
-  for (int i = threadIdx.x; i < g.nf * g.nby; i += blockDim.x) {
-    const int b = i / g.nby, r = i - b * g.nby, a = r - g.Ny;
-    const size_t o1 = (size_t)(a + g.Ny) * g.nbx + (b + g.Nx);
-    const size_t o2 = (size_t)(-a + g.Ny) * g.nbx + (-b + g.Nx);
-    float2 f1 = make_float2(0.f, 0.f), f2 = make_float2(0.f, 0.f);
-    for (int p = 0; p < nparts; ++p) {
-      f1 = cadd(f1, __ldg(p0 + p * nb2 + o1));
-      f2 = cadd(f2, __ldg(p0 + p * nb2 + o2));
-    }
-    To[i] = cscale(cadd(cconj(f1), f2), s);
-  }
-}
-
-// ---------------------------------------------------------------------------
 // vjp_source: dL/dJ_s = (1/G^2) sum_p gam(p) |e_s(p)|^2 / J_s, per (image, slice)
 // ---------------------------------------------------------------------------
 __host__ __device__ inline size_t gv_src_smem_elems(const GenGeom& g) {
@@ -599,20 +577,9 @@ int gen_launch_vjp_spectral(const GenGeom& g, const float2* band, int nparts, co
                             int nclips, const float2* H, const float* lam, int K, int nsets, int nsplit, float2* gam,
                             cudaStream_t st) {
   if (nclips <= 0) return KL_OK;
-  switch (g.RG) {
-    case 1: return launch_vspec_t<1>(g, band, nparts, gband, gparts, nclips, H, lam, K, nsets, nsplit, gam, st);
-    case 2: return launch_vspec_t<2>(g, band, nparts, gband, gparts, nclips, H, lam, K, nsets, nsplit, gam, st);
-    case 4: return launch_vspec_t<4>(g, band, nparts, gband, gparts, nclips, H, lam, K, nsets, nsplit, gam, st);
-    case 8: return launch_vspec_t<8>(g, band, nparts, gband, gparts, nclips, H, lam, K, nsets, nsplit, gam, st);
-  }
+  if (g.RG == 8) return launch_vspec_t<8>(g, band, nparts, gband, gparts, nclips, H, lam, K, nsets, nsplit, gam, st);
   set_error("gen_launch_vjp_spectral: unsupported spectral grid");
   return KL_ERR_UNSUPPORTED;
-}
-
-int gen_launch_gradT(const GenGeom& g, const float2* gam, int nclips, int nparts, float2* Tg, cudaStream_t st) {
-  if (nclips <= 0) return KL_OK;
-  k_gen_gradT<<<nclips, kT, 0, st>>>(gam, g, nparts, Tg);
-  return check_launch("k_gen_gradT");
 }
 
 int gen_launch_vjp_source(const GenGeom& g, const float2* band, int nparts, const float2* gband, int gparts,

@@ -311,131 +311,6 @@ __device__ __forceinline__ void field_rows(const SocsGeom& g, const float2* __re
 }
 
 // ---------------------------------------------------------------------------
-// Gam partial per (clip, set, kernel slice)
-// ---------------------------------------------------------------------------
-template <int RG>
-__global__ void __launch_bounds__(kThreads) k_vjp_spectral(const float2* __restrict__ partial,
-                                                           const float2* __restrict__ gpart,
-                                                           const SocsGeom g,
-                                                           const float2* __restrict__ H,
-                                                           const float* __restrict__ lam, int K,
-                                                           float2* __restrict__ gam_out) {
-  constexpr int G = 32 * RG, GP = G + 1;
-  extern __shared__ float4 smem4[];
-  const int nb2 = g.nby * g.nbx;
-  float2* Cm = reinterpret_cast<float2*>(smem4);    // [nby][nbx]
-  float2* Gacc = Cm + nb2;                           // [nby][nbx]
-  float2* E1 = Gacc + nb2;                           // [G][GP]  (G >= nby, nty)
-  float* gam = reinterpret_cast<float*>(E1 + G * GP);  // [G][GP]
-  // the band of dL/dI is read only while gam is made; the per-kernel stages
-  // then reuse its space (two CTAs per SM at 1024^2)
-  float2* Gb = reinterpret_cast<float2*>(gam + G * GP);  // [nty][W]
-  float2* Wg = Gb;                                        // [G][GP]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int clip = blockIdx.x, set = blockIdx.y, split = blockIdx.z;
-  const int nsets = gridDim.y, nsplit = gridDim.z;
-  const int img = clip * nsets + set;
-  const int k0 = (int)(((long long)K * split) / nsplit), k1 = (int)(((long long)K * (split + 1)) / nsplit);
-  const int br = (int)(__brev((unsigned)lane) >> 27);
-
-  load_band_v(partial, g, clip, Cm);
-  load_gbar(gpart, g, img, Gb);
-  for (int i = threadIdx.x; i < nb2; i += kThreads) Gacc[i] = make_float2(0.f, 0.f);
-  __syncthreads();
-  make_gamma<RG>(g, Gb, E1, gam, lane, warp);
-
-  WarpFFT<RG, +1> wi;
-  wi.init(lane);
-  const float invg2 = 1.0f / ((float)G * (float)G);
-  const size_t nbs = (size_t)nb2;
-  const float2* Hs = H + (size_t)set * K * nbs;
-  for (int k = k0; k < k1; ++k) {
-    const float2* Hk = Hs + (size_t)k * nbs;
-    const float lk = __ldg(lam + set * K + k) * invg2;
-    field_rows<RG>(g, Hk, Cm, E1, wi, lane, warp);
-    __syncthreads();
-    // stage 2: columns q -> e(p, q); w = conj(e) gam
-    for (int q = warp; q < G; q += kWarps) {
-      float2 vv[RG];
-#pragma unroll
-      for (int j = 0; j < RG; ++j) {
-        const int n = lane + 32 * j;
-        const int fy = n <= g.Ny ? n : (n >= G - g.Ny ? n - G : INT_MIN);
-        vv[j] = (fy != INT_MIN) ? E1[(fy + g.Ny) * GP + q] : make_float2(0.f, 0.f);
-      }
-      wi.run(vv, lane);
-#pragma unroll
-      for (int q1 = 0; q1 < RG; ++q1) {
-        const int p = q1 + RG * br;
-        Wg[p * GP + q] = cscale(cconj(vv[q1]), gam[p * GP + q]);
-      }
-    }
-    __syncthreads();
-    // stage 3: rows p, transform along x (sign +1), keep |fx| <= Nx -> E1[p][fx+Nx]
-    for (int p = warp; p < G; p += kWarps) {
-      float2 vv[RG];
-#pragma unroll
-      for (int j = 0; j < RG; ++j) vv[j] = Wg[p * GP + lane + 32 * j];
-      wi.run(vv, lane);
-#pragma unroll
-      for (int q1 = 0; q1 < RG; ++q1) {
-        const int bin = q1 + RG * br;
-        const int fx = bin <= G / 2 ? bin : bin - G;
-        if (fx >= -g.Nx && fx <= g.Nx) E1[p * GP + fx + g.Nx] = vv[q1];
-      }
-    }
-    __syncthreads();
-    // stage 4: columns fx, transform along y (sign +1), keep |fy| <= Ny -> B
-    for (int c = warp; c < g.nbx; c += kWarps) {
-      float2 vv[RG];
-#pragma unroll
-      for (int j = 0; j < RG; ++j) vv[j] = E1[(lane + 32 * j) * GP + c];
-      wi.run(vv, lane);
-#pragma unroll
-      for (int q1 = 0; q1 < RG; ++q1) {
-        const int bin = q1 + RG * br;
-        const int fy = bin <= G / 2 ? bin : bin - G;
-        if (fy >= -g.Ny && fy <= g.Ny) {
-          const int o = (fy + g.Ny) * g.nbx + c;
-          Gacc[o] = cfma(cscale(__ldg(Hk + o), lk), vv[q1], Gacc[o]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  float2* out = gam_out + (((size_t)clip * nsets + set) * nsplit + split) * nbs;
-  for (int i = threadIdx.x; i < nb2; i += kThreads) out[i] = Gacc[i];
-}
-
-// ---------------------------------------------------------------------------
-// Gam partials -> half-plane spectrum of dL/dm (for k_socs_inverse)
-// T[a][b] = (conj Gam[f] + Gam[-f]) / (Lx Ly), f = (a, b), |a| <= Ny, b <= Nx
-// ---------------------------------------------------------------------------
-__global__ void k_vjp_gradT(const float2* __restrict__ gam, const SocsGeom g, int nparts,
-                            float2* __restrict__ T) {
-  const int clip = blockIdx.x;
-  const size_t nbs = (size_t)g.nby * g.nbx;
-  const float2* p0 = gam + (size_t)clip * nparts * nbs;
-  const float s = 1.0f / ((float)g.Lx * (float)g.Ly);
-  float2* To = T + (size_t)clip * g.nty * g.ntx;
-  for (int i = threadIdx.x; i < g.nty * g.ntx; i += blockDim.x) {
-    const int r = i / g.ntx, b = i - r * g.ntx, a = r - 2 * g.Ny;
-    float2 v = make_float2(0.f, 0.f);
-    if (a >= -g.Ny && a <= g.Ny && b <= g.Nx) {
-      const size_t o1 = (size_t)(a + g.Ny) * g.nbx + (b + g.Nx);
-      const size_t o2 = (size_t)(-a + g.Ny) * g.nbx + (-b + g.Nx);
-      float2 f1 = make_float2(0.f, 0.f), f2 = make_float2(0.f, 0.f);
-      for (int p = 0; p < nparts; ++p) {
-        f1 = cadd(f1, p0[p * nbs + o1]);
-        f2 = cadd(f2, p0[p * nbs + o2]);
-      }
-      v = cscale(cadd(cconj(f1), f2), s);
-    }
-    To[i] = v;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // dL/dJ per (image, source slice): (1/G^2) sum_p gam |e_s|^2 / J_s
 // ---------------------------------------------------------------------------
 template <int RG>
@@ -535,11 +410,6 @@ int launch_vinv(const SocsGeom& g, const float2* tx, const float2* ty, const flo
   return check_launch("k_vjp_inverse");
 }
 
-size_t vjp_spectral_smem(const SocsGeom& g) {
-  const int G = g.G, GP = G + 1, nb2 = g.nby * g.nbx, W = 4 * g.Nx + 1;
-  const size_t shared = std::max((size_t)g.nty * W, (size_t)G * GP);  // dL/dI band, then Wg
-  return sizeof(float2) * ((size_t)2 * nb2 + (size_t)G * GP + shared) + sizeof(float) * (size_t)G * GP;
-}
 size_t vjp_source_smem(const SocsGeom& g) {
   const int G = g.G, GP = G + 1, nb2 = g.nby * g.nbx, W = 4 * g.Nx + 1;
   return sizeof(float2) * ((size_t)nb2 + (size_t)g.nty * W + (size_t)G * GP) +
@@ -573,30 +443,6 @@ int vjp_launch_inverse(const SocsGeom& g, const float2* tx, const float2* ty, co
 #undef KL_VINV
   set_error("vjp_launch_inverse: no kernel for this geometry");
   return KL_ERR_UNSUPPORTED;
-}
-
-int vjp_launch_spectral(const SocsGeom& g, const float2* partial, const float2* gpart, int nclips,
-                        const float2* H, const float* lam, int K, int nsets, int nsplit,
-                        float2* gam_out, cudaStream_t st) {
-  if (nclips <= 0) return KL_OK;
-  const size_t sm = vjp_spectral_smem(g);
-  if (g.G == 32) {
-    int rc = set_smem(k_vjp_spectral<1>, sm);
-    if (rc) return rc;
-    k_vjp_spectral<1><<<dim3(nclips, nsets, nsplit), kThreads, sm, st>>>(partial, gpart, g, H, lam, K, gam_out);
-  } else {
-    int rc = set_smem(k_vjp_spectral<2>, sm);
-    if (rc) return rc;
-    k_vjp_spectral<2><<<dim3(nclips, nsets, nsplit), kThreads, sm, st>>>(partial, gpart, g, H, lam, K, gam_out);
-  }
-  return check_launch("k_vjp_spectral");
-}
-
-int vjp_launch_gradT(const SocsGeom& g, const float2* gam, int nclips, int nparts, float2* T,
-                     cudaStream_t st) {
-  if (nclips <= 0) return KL_OK;
-  k_vjp_gradT<<<nclips, kThreads, 0, st>>>(gam, g, nparts, T);
-  return check_launch("k_vjp_gradT");
 }
 
 int vjp_launch_source(const SocsGeom& g, const float2* partial, const float2* gpart, int nimg,
