@@ -132,6 +132,21 @@ constexpr int kGenMaxSplit = 8;
 // the chunk twiddles of the row kernels are staged in shared memory up to 32 KB
 __host__ __device__ inline bool gen_t2_in_smem(const GenGeom& g) { return (size_t)g.nC * g.NBX * 8 <= 32 * 1024; }
 
+// Rows by matrix products (socs_rows.cu) instead of register FFTs of P points: their
+// time goes with the bins, that of the FFTs falls with P.  Measured at widths of 2001
+// (P = 1), 2002, 2004 and 1992 pixels, four clips of 1203 rows, 55 (synthesis of 8
+// images) and 28 bins (mask transform), us: synthesis 444, 212, 115, 63 by FFTs, 94 by
+// products; mask transform 150, 81, 55, 32 against 79; image, resist and transform of
+// dL/dI 601, 314, 170, 99 against 215.
+inline bool gen_direct_synth(const GenGeom& g) { return g.P <= 4 && g.ntx <= 112; }
+inline bool gen_direct_dft(const GenGeom& g) { return g.P <= 2 && g.ntx <= 112; }
+const float2* gen_roots_x(const GenGeom& g, const float2* tables);  // e^{+2 pi i m / Lx}
+int row_synth(const GenGeom& g, const float2* rlx, const float2* Q, int nrows, int nbins, float* out, cudaStream_t st);
+int row_dft(const GenGeom& g, const float2* rlx, const float* src, int nimg, int nbins, float2* R, cudaStream_t st);
+// row_dft of dL/dI, made from the images and targets; adds to loss[image]
+int row_dft_vjp(const GenGeom& g, const float2* rlx, const float* images, int nimg, int nbins, const float* targets,
+                int nsets, float alpha, float thr, double* loss, float2* R, cudaStream_t st);
+
 int gen_geometry(int Lx, int Ly, int Nx, int Ny, GenGeom* g);
 size_t gen_rowbins_bytes(const GenGeom& g, int nrows_img, int nbins);  // R / Q buffers
 size_t gen_band_bytes(const GenGeom& g, int n, int nparts, int nrows, int ncols);

@@ -361,8 +361,17 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
     return rc;
   if ((rc = kl::gen_launch_colinv(g, p->gtab, p->T, nimg, 2 * g.Ny, g.ntx, p->Q, st))) return rc;
   KL_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(double) * (size_t)nimg, st));
-  if ((rc = kl::gen_launch_rowvjp(g, p->gtab, p->Q, nimg, p->nsets, targets, alpha, threshold, images, loss, st)))
-    return rc;
+  // image, then dL/dI's row bins from it; without a place for the image (no output
+  // for it, several images per clip) both in one kernel.  The gradient is written last
+  float* im = images ? images : p->nsets == 1 ? grad : nullptr;
+  if (kl::gen_direct_dft(g) && im) {
+    const float2* rlx = kl::gen_roots_x(g, p->gtab);
+    if ((rc = kl::row_synth(g, rlx, p->Q, nimg * g.Ly, g.ntx, im, st))) return rc;
+    rc = kl::row_dft_vjp(g, rlx, im, nimg, g.ntx, targets, p->nsets, alpha, threshold, loss, p->Q, st);
+  } else {
+    rc = kl::gen_launch_rowvjp(g, p->gtab, p->Q, nimg, p->nsets, targets, alpha, threshold, images, loss, st);
+  }
+  if (rc) return rc;
   if ((rc = kl::gen_launch_colfwd(g, p->gtab, p->Q, nimg, g.ntx, 2 * g.Ny, 1.0f, gparts, p->gband, st))) return rc;
   rc = kl::adjoint_core(p->sg)
            ? kl::adjoint_launch(p->sg, p->band, nparts, 1.0f, p->gband, gparts, nimg, p->HT, p->lam, p->K, p->nsets, ns_adj,

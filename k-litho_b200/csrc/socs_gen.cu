@@ -120,7 +120,8 @@ size_t gen_band_bytes(const GenGeom& g, int n, int nparts, int nrows, int ncols)
   (void)g;
   return sizeof(float2) * (size_t)n * nparts * nrows * ncols;
 }
-size_t gen_table_elems(const GenGeom& g) { return off_rly(g) + (size_t)g.Ly; }
+size_t gen_table_elems(const GenGeom& g) { return off_rly(g) + (size_t)g.Ly + g.Lx; }
+const float2* gen_roots_x(const GenGeom& g, const float2* tables) { return tables + off_rly(g) + g.Ly; }
 
 int gen_choose_split(const GenGeom& g, int nimg, int K) {
   // kernel slices per image: the count whose CTAs fill the GPU's resident
@@ -153,10 +154,10 @@ int gen_choose_parts(const GenGeom& g, int n, int ncols) {
 }
 
 // twb[b][l] = twl[l][b] = e^{+2 pi i b l / Lx}; tw2[c][b] = e^{+2 pi i b 32 c / Lx};
-// rly[m] = e^{+2 pi i m / Ly}
+// rly[m] = e^{+2 pi i m / Ly}; rlx[m] = e^{+2 pi i m / Lx}
 __global__ void k_gen_tables(const GenGeom g, float2* __restrict__ t) {
   const size_t n1 = (size_t)g.NBX * 32, n2 = (size_t)g.nC * g.NBX;
-  const size_t n = off_rly(g) + g.Ly;
+  const size_t n = off_rly(g) + g.Ly + g.Lx;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
     float2 v;
     if (i < n1) {
@@ -170,8 +171,10 @@ __global__ void k_gen_tables(const GenGeom g, float2* __restrict__ t) {
       const size_t j = i - 2 * n1;
       const int c = (int)(j / g.NBX), b = (int)(j % g.NBX);
       v = expi2pi_frac((long long)b * 32 * c, g.Lx);
-    } else {
+    } else if (i < off_rly(g) + g.Ly) {
       v = expi2pi_frac((long long)(i - off_rly(g)), g.Ly);
+    } else {
+      v = expi2pi_frac((long long)(i - off_rly(g) - g.Ly), g.Lx);
     }
     t[i] = v;
   }
@@ -653,6 +656,7 @@ int launch_rowinv_t(const GenGeom& g, const float2* tables, const float2* Q, int
 int gen_launch_rowfwd(const GenGeom& g, const float2* tables, const float* src, int nrows, float2* R,
                       cudaStream_t st) {
   if (nrows <= 0) return KL_OK;
+  if (gen_direct_dft(g)) return row_dft(g, gen_roots_x(g, tables), src, nrows / g.Ly, g.nf, R, st);
   switch (g.Pf) {
     case 1: return launch_rowfwd_t<1>(g, tables, src, nrows, g.nf, R, st);
     case 2: return launch_rowfwd_t<2>(g, tables, src, nrows, g.nf, R, st);
@@ -713,6 +717,7 @@ int gen_launch_rowinv(const GenGeom& g, const float2* tables, const float2* Q, i
                       cudaStream_t st) {
   if (nimg <= 0) return KL_OK;
   const int nrows = nimg * g.Ly;
+  if (gen_direct_synth(g)) return row_synth(g, gen_roots_x(g, tables), Q, nrows, nbins, images, st);
   switch (g.P) {
     case 1: return launch_rowinv_t<1>(g, tables, Q, nrows, nbins, images, st);
     case 2: return launch_rowinv_t<2>(g, tables, Q, nrows, nbins, images, st);
