@@ -35,7 +35,7 @@ namespace kl {
 
 namespace {
 constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
+constexpr int kSMs = 148;
 
 __host__ __device__ inline int pow2_at_least(int v) {
   int p = 1;
@@ -148,8 +148,8 @@ int socs_build_tables(const SocsGeom& g, float2* tx, float2* ty, cudaStream_t st
 // ---------------------------------------------------------------------------
 // 1. forward: mask rows -> per-strip partial band spectra
 // ---------------------------------------------------------------------------
-template <int P, int V, int NFM, int RJ>
-__global__ void __launch_bounds__(kThreads) k_socs_forward(const float* __restrict__ masks,
+template <int P, int V, int NFM, int RJ, int NT>
+__global__ void __launch_bounds__(NT) k_socs_forward(const float* __restrict__ masks,
                                                            const SocsGeom g,
                                                            const float2* __restrict__ tx,
                                                            const float2* __restrict__ ty,
@@ -162,12 +162,12 @@ __global__ void __launch_bounds__(kThreads) k_socs_forward(const float* __restri
   const int s = blockIdx.x, clip = blockIdx.y;
   const float* mask = masks + (size_t)clip * g.Lx * g.Ly;
 
-  for (int i = threadIdx.x; i < NFM * V; i += kThreads) twf[i] = __ldg(tx + i);
+  for (int i = threadIdx.x; i < NFM * V; i += NT) twf[i] = __ldg(tx + i);
   dep_wait();
   dep_launch();
   __syncthreads();
 
-  for (int jj = warp; jj < J; jj += kWarps) {
+  for (int jj = warp; jj < J; jj += (NT / 32)) {
     const float* row = mask + (size_t)(s + g.nS * jj) * (V * P);
     float acc[2 * NFM];
 #pragma unroll
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) k_socs_forward(const float* __restri
   wf.init(lane);
   const int br = (int)(__brev((unsigned)lane) >> 27);
   const float2* tys = ty + (size_t)s * g.nty + 2 * g.Ny;  // e^{+2 pi i a s/Ly} at [a]
-  for (int fx = warp; fx < g.nf; fx += kWarps) {
+  for (int fx = warp; fx < g.nf; fx += (NT / 32)) {
     float2 vv[RJ];
 #pragma unroll
     for (int j = 0; j < RJ; ++j) vv[j] = rowbuf[(lane + 32 * j) * NFM + fx];
@@ -236,8 +236,8 @@ __device__ __forceinline__ void load_band(const float2* __restrict__ partial, co
 // ---------------------------------------------------------------------------
 // 3. inverse: intensity spectrum -> image rows
 // ---------------------------------------------------------------------------
-template <int P, int V, int NBM, int RJ>
-__global__ void __launch_bounds__(kThreads) k_socs_inverse(const float2* __restrict__ T,
+template <int P, int V, int NBM, int RJ, int NT>
+__global__ void __launch_bounds__(NT) k_socs_inverse(const float2* __restrict__ T,
                                                            const SocsGeom g,
                                                            const float2* __restrict__ tx,
                                                            const float2* __restrict__ ty,
@@ -259,12 +259,12 @@ __global__ void __launch_bounds__(kThreads) k_socs_inverse(const float2* __restr
   // once per CTA: the x twiddles, the zero columns b >= ntx of the row
   // coefficients and the image's band spectrum
 #pragma unroll 4
-  for (int i = threadIdx.x; i < NBM * V; i += kThreads) twi[i] = __ldg(tx + i);
-  for (int i = threadIdx.x; i < J * QP; i += kThreads) Qs[i] = make_float2(0.f, 0.f);
+  for (int i = threadIdx.x; i < NBM * V; i += NT) twi[i] = __ldg(tx + i);
+  for (int i = threadIdx.x; i < J * QP; i += NT) Qs[i] = make_float2(0.f, 0.f);
   dep_wait();
   dep_launch();
 #pragma unroll 4
-  for (int i = threadIdx.x; i < (int)tsz; i += kThreads) Ts[i] = __ldg(Ti + i);
+  for (int i = threadIdx.x; i < (int)tsz; i += NT) Ts[i] = __ldg(Ti + i);
   float2 ph_next = make_float2(0.f, 0.f);
   if (threadIdx.x < g.nty) ph_next = __ldg(ty + (size_t)s0 * g.nty + threadIdx.x);
   __syncthreads();
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kThreads) k_socs_inverse(const float2* __restr
     }
     __syncthreads();
     // rows of the strip: Q[y = s + nS j][b] = sum_a T[a][b] e^{2 pi i a y / Ly}
-    for (int b = warp; b < g.ntx; b += kWarps) {
+    for (int b = warp; b < g.ntx; b += (NT / 32)) {
       float2 vv[RJ];
 #pragma unroll
       for (int j = 0; j < RJ; ++j) {
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(kThreads) k_socs_inverse(const float2* __restr
     }
     __syncthreads();
 
-    for (int jj = warp; jj < J; jj += kWarps) {
+    for (int jj = warp; jj < J; jj += (NT / 32)) {
       float* row = out + (size_t)(s + g.nS * jj) * (V * P);
       const float2* q = Qs + jj * QP;
 #pragma unroll 1
@@ -406,11 +406,14 @@ template <int P, int V, int NFM, int RJ>
 int launch_fwd(const SocsGeom& g, const float2* tx, const float2* ty, const float* masks,
                int nclips, float2* partial, cudaStream_t st) {
   size_t sm = sizeof(float2) * ((size_t)NFM * V + (size_t)32 * RJ * NFM);
-  auto kern = k_socs_forward<P, V, NFM, RJ>;
-  int rc = set_smem(kern, sm);
-  if (rc) return rc;
-  KL_CUDA_TRY(launch_dependent(kern, dim3(g.nS, nclips), kThreads, sm, st, masks, g, tx, ty, partial));
-  return KL_OK;
+  auto launch = [&](auto kern, int threads) -> int {
+    if (int rc = set_smem(kern, sm)) return rc;
+    KL_CUDA_TRY(launch_dependent(kern, dim3(g.nS, nclips), threads, sm, st, masks, g, tx, ty, partial));
+    return KL_OK;
+  };
+  // a strip's rows on twice the warps where the strips leave SMs idle
+  if ((long long)g.nS * nclips <= kSMs) return launch(k_socs_forward<P, V, NFM, RJ, 2 * kThreads>, 2 * kThreads);
+  return launch(k_socs_forward<P, V, NFM, RJ, kThreads>, kThreads);
 }
 
 template <int P, int V, int NBM, int RJ>
@@ -418,9 +421,6 @@ int launch_inv(const SocsGeom& g, const float2* tx, const float2* ty, const floa
                float* images, cudaStream_t st, int spc) {
   size_t sm = sizeof(float2) * ((size_t)NBM * V + (size_t)32 * RJ * (NBM + 1) +
                                 (size_t)g.nty * g.ntx + g.nty);
-  auto kern = k_socs_inverse<P, V, NBM, RJ>;
-  int rc = set_smem(kern, sm);
-  if (rc) return rc;
   // strips per CTA: the image's spectrum and the twiddle table are loaded once
   // per CTA, so give each CTA several strips while keeping >= 4 CTAs per SM
   if (spc <= 0) {
@@ -428,8 +428,14 @@ int launch_inv(const SocsGeom& g, const float2* tx, const float2* ty, const floa
     while (spc < 8 && spc * 2 <= g.nS && (long long)nimg * ((g.nS + 2 * spc - 1) / (2 * spc)) >= 4 * 148) spc *= 2;
   }
   spc = spc < g.nS ? spc : g.nS;
-  KL_CUDA_TRY(launch_dependent(kern, dim3((g.nS + spc - 1) / spc, nimg), kThreads, sm, st, T, g, tx, ty, spc, images));
-  return KL_OK;
+  const dim3 grid((g.nS + spc - 1) / spc, nimg);
+  auto launch = [&](auto kern, int threads) -> int {
+    if (int rc = set_smem(kern, sm)) return rc;
+    KL_CUDA_TRY(launch_dependent(kern, grid, threads, sm, st, T, g, tx, ty, spc, images));
+    return KL_OK;
+  };
+  if ((long long)grid.x * nimg <= kSMs) return launch(k_socs_inverse<P, V, NBM, RJ, 2 * kThreads>, 2 * kThreads);
+  return launch(k_socs_inverse<P, V, NBM, RJ, kThreads>, kThreads);
 }
 
 }  // namespace
