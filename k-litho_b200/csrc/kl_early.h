@@ -3,7 +3,8 @@
 
 namespace kl {
 // whether this thread's launches may start ahead: not while stage events are
-// recorded between the kernels, nor in concurrent branches
+// recorded between the kernels, in concurrent branches, or where tables and kernels
+// are not a plan's
 inline thread_local bool t_early_launch = true;
 // sets it for a scope; a scope inside one that turned it off cannot turn it on
 struct EarlyLaunch {

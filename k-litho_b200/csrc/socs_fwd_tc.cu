@@ -5,7 +5,7 @@
 // each strip s of J rows (y = s + nS j) the partial band spectrum
 //     D_s[fy][fx] = sum_j e^{-2 pi i fy (s + nS j)/Ly} R[s + nS j][fx],
 //     R[y][fx]    = sum_x m[y][x] e^{-2 pi i fx x / Lx},   0 <= fx <= Nx,
-// of which k_socs_spectral sums the strips.  The row DFT R is a matrix
+// of which the spectral core sums the strips.  The row DFT R is a matrix
 // product per tile of 128 rows (128/J strips): R = M . BT with the mask block
 // M (FP16 hi/lo halves in TMEM: mask values must lie within +-2^15) and the
 // plan's transposed cos/sin basis BT (FP16 hi/lo, L2-resident), accumulated

@@ -22,6 +22,7 @@
 #include <mutex>
 #include <string>
 
+#include "kl_early.h"
 #include "kl_internal.h"
 
 namespace {
@@ -101,7 +102,10 @@ extern "C" int kl_socs_forward_noalloc(const float* masks_dev, int nclips, int L
   const size_t b_tx = up256(sizeof(float2) * kl::socs_table_x_elems(g));
   const size_t b_ty = up256(sizeof(float2) * kl::socs_table_y_elems(g));
   const size_t b_part = up256(kl::socs_partial_bytes(g, nclips));
-  const size_t b_T = up256(sizeof(float2) * (size_t)nclips * g.nty * g.ntx);
+  // a call's budget counts the spectra of the kernel slices (up to 8) of few clips
+  int slices = 1;
+  while (slices < 8 && nclips * slices < 2 * 148 && nk / (2 * slices) >= 3) slices *= 2;
+  const size_t b_T = up256(sizeof(float2) * (size_t)nclips * slices * g.nty * g.ntx);
   const size_t need = b_tx + b_ty + b_part + b_T;
   // what the spectral core's CTAs hold of an image, and its counters, pass through
   // the image buffer: it is written only afterwards
@@ -127,6 +131,9 @@ extern "C" int kl_socs_forward_noalloc(const float* masks_dev, int nclips, int L
   unsigned* done = reinterpret_cast<unsigned*>((reinterpret_cast<uintptr_t>(images_dev) + 255) & ~uintptr_t(255));
   float2* core = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(done) + b_cnt);
   cudaStream_t st = (cudaStream_t)stream;
+  // one kernel after the other: unlike a plan's, the twiddle tables and kernels read
+  // ahead of a predecessor's end would be that predecessor's or the caller's output
+  const kl::EarlyLaunch in_order(false);
   if ((rc = kl::socs_build_tables(g, tx, ty, st))) return rc;
   if ((rc = kl::socs_launch_forward(g, tx, ty, masks_dev, nclips, partial, st))) return rc;
   KL_CUDA_TRY(cudaMemsetAsync(done, 0, sizeof(unsigned) * nclips, st));
