@@ -174,17 +174,17 @@ __device__ __forceinline__ void rdft_reg(const float (&v)[P], float2 (&S)[P / 2 
 #pragma unroll
   for (int m = 0; m < H; ++m) z[m] = make_float2(v[2 * m], v[2 * m + 1]);
   fft_reg<H, -1>(z);
-  // S[k] = (Z[k] + conj Z[H-k])/2 - i e^{-2 pi i k/P} (Z[k] - conj Z[H-k])/2
+  // S[k] = (Z[k] + conj Z[H-k])/2 - i e^{-2 pi i k/P} (Z[k] - conj Z[H-k])/2; H-k has
+  // the conjugates of both terms
+  S[0] = make_float2(z[0].x + z[0].y, 0.f);
+  S[H] = make_float2(z[0].x - z[0].y, 0.f);
+  if constexpr (H > 1) S[H / 2] = cconj(z[H / 2]);
 #pragma unroll
-  for (int k = 0; k <= H; ++k) {
-    float2 a = z[k % H];
-    float2 b = cconj(z[(H - k) % H]);
-    float2 ev = cscale(cadd(a, b), 0.5f);
-    float2 od = cscale(csub(a, b), 0.5f);
-    float2 w = tw_const<P, -1>(k);
-    // -i * w * od
-    float2 t = cmul(w, od);
-    S[k] = make_float2(ev.x + t.y, ev.y - t.x);
+  for (int k = 1; k < H / 2; ++k) {
+    const float2 ev = cadd(z[k], cconj(z[H - k]));
+    const float2 t = cmul(cscale(tw_const<P, -1>(k), 0.5f), csub(z[k], cconj(z[H - k])));
+    S[k] = make_float2(fmaf(0.5f, ev.x, t.y), fmaf(0.5f, ev.y, -t.x));
+    S[H - k] = make_float2(fmaf(0.5f, ev.x, -t.y), fmaf(-0.5f, ev.y, -t.x));
   }
 }
 
@@ -232,14 +232,16 @@ __device__ __forceinline__ void c2r_half(const float2 (&Y)[P / 2 + 1], float (&o
   } else {
     constexpr int H = P / 2;
     float2 x[H];
+    // x[k] = fe + i fo from F[k] and F[k+H] of the Hermitian spectrum F[k] = Y[k]/2
+    // (0 < k < H), F[P-k] = conj F[k]; H-k has the conjugates of both
+    x[0] = make_float2(Y[0].x + Y[H].x, Y[0].x - Y[H].x);
+    if constexpr (H > 1) x[H / 2] = cconj(Y[H / 2]);
 #pragma unroll
-    for (int k = 0; k < H; ++k) {
-      // F[k] and F[k+H] of the Hermitian spectrum F[k] = Y[k]/2 (0<k<H), F[P-k] = conj F[k]
-      const float2 a = k == 0 ? make_float2(Y[0].x, 0.f) : cscale(Y[k], 0.5f);
-      const float2 b = k == 0 ? make_float2(Y[H].x, 0.f) : cscale(cconj(Y[H - k]), 0.5f);
-      const float2 fe = cadd(a, b);
-      const float2 fo = cmul(csub(a, b), tw_const<P, +1>(k));
-      x[k] = make_float2(fe.x - fo.y, fe.y + fo.x);
+    for (int k = 1; k < H / 2; ++k) {
+      const float2 fe = cadd(Y[k], cconj(Y[H - k]));
+      const float2 fo = cmul(csub(Y[k], cconj(Y[H - k])), cscale(tw_const<P, +1>(k), 0.5f));
+      x[k] = make_float2(fmaf(0.5f, fe.x, -fo.y), fmaf(0.5f, fe.y, fo.x));
+      x[H - k] = make_float2(fmaf(0.5f, fe.x, fo.y), fmaf(-0.5f, fe.y, fo.x));
     }
     fft_reg<H, +1>(x);
 #pragma unroll

@@ -36,6 +36,7 @@
 #include "kl_device.cuh"
 #include "kl_internal.h"
 #include "kl_launch.cuh"
+#include "row_fold.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -599,6 +600,47 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* __restrict__ Q,
   }
 }
 
+// The same for P >= 8 with the twiddles factored (row_fold.cuh).
+template <int P, bool SM>
+__global__ void __launch_bounds__(kT) k_gen_rowinv_fold(const float2* __restrict__ Q, int nbins, int nrows,
+                                                        const GenGeom g, const float2* __restrict__ rlx,
+                                                        float* __restrict__ out) {
+  extern __shared__ float4 smem4[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2* qs = reinterpret_cast<float2*>(smem4) + warp * g.NBX;  // this warp's row
+  float2* tb = reinterpret_cast<float2*>(smem4) + kW * g.NBX;
+  const int V = g.V, nch = (V + 31) / 32;
+  if (SM) row_fold_tables<P>(rlx, V, threadIdx.x, kT, tb);
+  __syncthreads();
+  dep_wait();
+  dep_launch();
+  const int nbp = (nbins + P - 1) / P * P;
+  float2 qn[4];
+  const int row0 = blockIdx.x * kW + warp, rstep = gridDim.x * kW;
+  if (row0 < nrows) gen_load_qrow(Q + (size_t)row0 * nbins, nbins, lane, qn);
+  for (int row = row0; row < nrows; row += rstep) {
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (lane + 32 * t < nbp) qs[lane + 32 * t] = qn[t];
+    __syncwarp();
+    if (row + rstep < nrows) gen_load_qrow(Q + (size_t)(row + rstep) * nbins, nbins, lane, qn);
+    float* orow = out + (size_t)row * g.Lx;
+#pragma unroll 1
+    for (int c = 0; c < nch; ++c) {
+      const int lp = lane + 32 * c;
+      float2 Y[P / 2 + 1];
+      row_fold<P, SM>(qs, nbins, SM ? tb : rlx, V, lp < V ? lp : 0, Y);
+      float o[P];
+      c2r_half<P>(Y, o);
+      if (lp < V) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) __stcs(orow + lp + V * i, o[i]);
+      }
+    }
+  }
+}
+
 // centred FT_r2c band: M(ky,kx) = D(ky,kx) e^{-2 pi i (ky yh/Ly + kx xh/Lx)}
 __global__ void k_gen_bandout(const float2* __restrict__ band, int nparts, const GenGeom g,
                               float2* __restrict__ out) {
@@ -648,6 +690,20 @@ int launch_rowinv_t(const GenGeom& g, const float2* tables, const float2* Q, int
   int rc = set_smem(kern, sm);
   if (rc) return rc;
   KL_CUDA_TRY(launch_dependent(kern, row_grid(nrows, 8), kT, sm, st, Q, nbins, nrows, g, tables, out));
+  return KL_OK;
+}
+
+template <int P>
+int launch_rowinv_fold(const GenGeom& g, const float2* tables, const float2* Q, int nrows, int nbins, float* out,
+                       cudaStream_t st) {
+  const bool in_smem = row_fold_in_smem(P, g.V);
+  const size_t sm = sizeof(float2) * ((size_t)kW * g.NBX + (in_smem ? row_fold_elems(P, g.V) : 0));
+  auto kern = in_smem ? k_gen_rowinv_fold<P, true> : k_gen_rowinv_fold<P, false>;
+  int rc = set_smem(kern, sm);
+  if (rc) return rc;
+  // 2, 3, 4, 6 and 8 CTAs per SM: 7 x 2 images of 1000 x 744 (P = 8) 99, 97, 94, 94, 95 us
+  // a call, 20 of 4096^2 (P = 64) 829, 837, 828, 826, 827
+  KL_CUDA_TRY(launch_dependent(kern, row_grid(nrows, 4), kT, sm, st, Q, nbins, nrows, g, gen_roots_x(g, tables), out));
   return KL_OK;
 }
 
@@ -722,10 +778,10 @@ int gen_launch_rowinv(const GenGeom& g, const float2* tables, const float2* Q, i
     case 1: return launch_rowinv_t<1>(g, tables, Q, nrows, nbins, images, st);
     case 2: return launch_rowinv_t<2>(g, tables, Q, nrows, nbins, images, st);
     case 4: return launch_rowinv_t<4>(g, tables, Q, nrows, nbins, images, st);
-    case 8: return launch_rowinv_t<8>(g, tables, Q, nrows, nbins, images, st);
-    case 16: return launch_rowinv_t<16>(g, tables, Q, nrows, nbins, images, st);
-    case 32: return launch_rowinv_t<32>(g, tables, Q, nrows, nbins, images, st);
-    case 64: return launch_rowinv_t<64>(g, tables, Q, nrows, nbins, images, st);
+    case 8: return launch_rowinv_fold<8>(g, tables, Q, nrows, nbins, images, st);
+    case 16: return launch_rowinv_fold<16>(g, tables, Q, nrows, nbins, images, st);
+    case 32: return launch_rowinv_fold<32>(g, tables, Q, nrows, nbins, images, st);
+    case 64: return launch_rowinv_fold<64>(g, tables, Q, nrows, nbins, images, st);
   }
   set_error("gen_launch_rowinv: unsupported row transform length");
   return KL_ERR_UNSUPPORTED;

@@ -30,6 +30,7 @@
 
 #include "kl_device.cuh"
 #include "kl_internal.h"
+#include "row_fold.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -66,9 +67,11 @@ int check_launch(const char* what) {
 // ---------------------------------------------------------------------------
 // row_vjp: Q rows -> image rows, resist, loss, dL/dI row DFT (written over Q)
 // ---------------------------------------------------------------------------
-template <int PF>
+// PF >= 8: twiddles factored (row_fold.cuh), FOLD its tables in shared memory.
+template <int PF, bool FOLD>
 __global__ void __launch_bounds__(kT, 2) k_gen_rowvjp(float2* __restrict__ Q, const GenGeom g,
-                                                   const float2* __restrict__ tables, int nsets,
+                                                   const float2* __restrict__ tables,
+                                                   const float2* __restrict__ rlx, int nsets,
                                                    const float* __restrict__ targets, float alpha, float thr,
                                                    float* __restrict__ images, double* __restrict__ loss) {
   constexpr int HS = PF / 2 + 1;
@@ -76,15 +79,20 @@ __global__ void __launch_bounds__(kT, 2) k_gen_rowvjp(float2* __restrict__ Q, co
   __shared__ double s_loss[kW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int NBX = g.NBX, ntx = g.ntx;
-  float2* tb = reinterpret_cast<float2*>(smem4);  // [NBX][32] e^{+2 pi i b l / Lx}
-  float2* tl = tb + NBX * 32;                      // [32][NBX] the same, transposed
-  float2* qc = tl + NBX * 32 + warp * NBX;         // [NBX]
-  float2* sb = tl + NBX * 32 + kW * NBX + warp * HS * 33;  // [HS][33]
-  float2* t2s = tl + NBX * 32 + kW * NBX + kW * HS * 33;   // [nC][NBX] chunk twiddles, when they fit
+  float2* tl = reinterpret_cast<float2*>(smem4);  // [32][NBX] e^{+2 pi i b l / Lx}
+  float2* qc = tl + NBX * 32 + warp * NBX;        // [NBX]
+  float2* tb = tl + NBX * 32 + kW * NBX;          // PF >= 8: row_fold's; else tl transposed
+  float2* sb = tb + (PF < 8 ? NBX * 32 : FOLD ? row_fold_elems(PF, g.Vf) : 0);
+  float2* t2s = sb + kW * HS * 33;  // [nC][NBX] chunk twiddles, when they fit
+  sb += warp * HS * 33;             // [HS][33]
   const int Lx = g.Lx, Ly = g.Ly, V = g.Vf, nch = (V + 31) / 32;
   const bool t2_shared = gen_t2_in_smem(g);
   const float2* tw2 = t2_shared ? t2s : tables + off_tw2(g);
-  for (int i = threadIdx.x; i < 64 * NBX; i += kT) tb[i] = __ldg(tables + i);
+  for (int i = threadIdx.x; i < 32 * NBX; i += kT) tl[i] = __ldg(tables + 32 * NBX + i);
+  if constexpr (PF < 8)
+    for (int i = threadIdx.x; i < 32 * NBX; i += kT) tb[i] = __ldg(tables + i);
+  else if (FOLD)
+    row_fold_tables<PF>(rlx, V, threadIdx.x, kT, tb);
   if (t2_shared)
     for (int i = threadIdx.x; i < nch * NBX; i += kT) t2s[i] = __ldg(tables + off_tw2(g) + i);
   __syncthreads();
@@ -110,6 +118,12 @@ __global__ void __launch_bounds__(kT, 2) k_gen_rowvjp(float2* __restrict__ Q, co
 #pragma unroll
     for (int t = 0; t < 4; ++t) acc[t] = make_float2(0.f, 0.f);
     float rsum = 0.f;
+    if constexpr (PF >= 8) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (lane + 32 * t < nbp) qc[lane + 32 * t] = q[t];
+      __syncwarp();
+    }
 #pragma unroll 1
     for (int c = 0; c < nch; ++c) {
       const int lp = lane + 32 * c;
@@ -117,26 +131,30 @@ __global__ void __launch_bounds__(kT, 2) k_gen_rowvjp(float2* __restrict__ Q, co
       float tg[PF];
 #pragma unroll
       for (int i = 0; i < PF; ++i) tg[i] = lp < V ? __ldcs(trow + lp + V * i) : 0.f;
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int b = lane + 32 * t;
-        if (b < nbp) qc[b] = b < ntx ? cmul(q[t], tw2[(size_t)c * NBX + b]) : make_float2(0.f, 0.f);
-      }
-      __syncwarp();
       float2 Y[HS];
+      if constexpr (PF >= 8) {
+        row_fold<PF, FOLD>(qc, ntx, FOLD ? tb : rlx, V, lp < V ? lp : 0, Y);
+      } else {
 #pragma unroll
-      for (int k = 0; k < HS; ++k) Y[k] = make_float2(0.f, 0.f);
+        for (int t = 0; t < 4; ++t) {
+          const int b = lane + 32 * t;
+          if (b < nbp) qc[b] = b < ntx ? cmul(q[t], tw2[(size_t)c * NBX + b]) : make_float2(0.f, 0.f);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < HS; ++k) Y[k] = make_float2(0.f, 0.f);
 #pragma unroll 1
-      for (int b0 = 0; b0 < nbp; b0 += PF) {
+        for (int b0 = 0; b0 < nbp; b0 += PF) {
 #pragma unroll
-        for (int k = 0; k < PF; ++k) {
-          const float2 q = qc[b0 + k];
-          const float2 w = tb[(b0 + k) * 32 + lane];
-          if (2 * k <= PF) {
-            Y[k] = cfma(q, w, Y[k]);
-          } else {
-            Y[PF - k].x = fmaf(q.x, w.x, fmaf(-q.y, w.y, Y[PF - k].x));
-            Y[PF - k].y = fmaf(-q.x, w.y, fmaf(-q.y, w.x, Y[PF - k].y));
+          for (int k = 0; k < PF; ++k) {
+            const float2 q = qc[b0 + k];
+            const float2 w = tb[(b0 + k) * 32 + lane];
+            if (2 * k <= PF) {
+              Y[k] = cfma(q, w, Y[k]);
+            } else {
+              Y[PF - k].x = fmaf(q.x, w.x, fmaf(-q.y, w.y, Y[PF - k].x));
+              Y[PF - k].y = fmaf(-q.x, w.y, fmaf(-q.y, w.x, Y[PF - k].y));
+            }
           }
         }
       }
@@ -500,15 +518,20 @@ namespace {
 template <int PF>
 int launch_rowvjp_t(const GenGeom& g, const float2* tables, float2* Q, int nimg, int nsets, const float* targets,
                     float alpha, float thr, float* images, double* loss, cudaStream_t st) {
-  const size_t sm = sizeof(float2) * ((size_t)64 * g.NBX + (size_t)kW * g.NBX + (size_t)kW * (PF / 2 + 1) * 33 +
+  const bool fold = PF >= 8 && row_fold_in_smem(PF, g.Vf);
+  const size_t sm = sizeof(float2) * ((size_t)32 * g.NBX + (size_t)kW * g.NBX + (size_t)kW * (PF / 2 + 1) * 33 +
+                                      (PF < 8 ? (size_t)32 * g.NBX : fold ? row_fold_elems(PF, g.Vf) : 0) +
                                       (gen_t2_in_smem(g) ? (size_t)g.nC * g.NBX : 0));
-  auto kern = k_gen_rowvjp<PF>;
+  auto kern = k_gen_rowvjp<PF, false>;
+  if constexpr (PF >= 8)
+    if (fold) kern = k_gen_rowvjp<PF, true>;
   int rc = set_smem(kern, sm);
   if (rc) return rc;
   // about four CTAs per SM over the whole batch, each on rows of one image
   int bx = (4 * kSMs + nimg - 1) / nimg;
   bx = std::max(1, std::min(bx, (g.Ly + kW - 1) / kW));
-  kern<<<dim3(bx, nimg), kT, sm, st>>>(Q, g, tables, nsets, targets, alpha, thr, images, loss);
+  kern<<<dim3(bx, nimg), kT, sm, st>>>(Q, g, tables, gen_roots_x(g, tables), nsets, targets, alpha, thr,
+                                          images, loss);
   return check_launch("k_gen_rowvjp");
 }
 
