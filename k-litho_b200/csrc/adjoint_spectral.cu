@@ -56,11 +56,13 @@ struct AdjSmem {
 // gam of one image at the grid columns of residue c, a CTA each, for the adjoint
 // kernel's column threads: gamma[img][c][r][i][lane], i the transform's output order.
 // Once per image instead of once per kernel slice, and out of that kernel's code (it
-// took 25 us of a single small clip's adjoint there).
+// took 25 us of a single small clip's adjoint there).  A few CTAs read every partial
+// band, so the loads in flight bound it: four images at G = 128 (16 bands of 96 KB each)
+// 33 us with 16 float2 per thread, 23 with 32.
 template <int RG>
 __global__ void __launch_bounds__(512) k_adjoint_gamma(const float2* __restrict__ gband, int gparts, const SpecGeom g,
                                                        float* __restrict__ gamma) {
-  constexpr int G = 32 * RG, kT = 512, kAhead = 8, kEach = 2;
+  constexpr int G = 32 * RG, kT = 512, kAhead = 16, kEach = 2;
   extern __shared__ float4 smem4[];
   float2* Gs = reinterpret_cast<float2*>(smem4);  // [nty][ntx] Gb for gx >= 0; then [nty][33] its rows along x
   __shared__ float2 roots[G];
@@ -408,7 +410,8 @@ int launch_adjoint(const SpecGeom& g, const float2* band, int nparts, float scal
 }
 
 // T(a, b) = (conj Gam[a][b] + Gam[-a][-b]) / (Lx Ly) for |a| <= Ny, 0 <= b <= Nx, zero in
-// the rest of [-ay, ay] x [0, nb): the half-plane spectrum of dL/dm
+// the rest of [-ay, ay] x [0, nb): the half-plane spectrum of dL/dm.  32 loads in flight
+// per thread: 32 shares of four images 10 us (31 with 16)
 __global__ void __launch_bounds__(128) k_adjoint_grad(const float2* __restrict__ gam, const SpecGeom g, int nparts, int ay,
                                                       int nb, int sa, int sb, float2* __restrict__ T) {
   dep_wait();
@@ -421,7 +424,7 @@ __global__ void __launch_bounds__(128) k_adjoint_grad(const float2* __restrict__
   if (a >= -g.Ny && a <= g.Ny && b <= g.Nx) {
     const float2* p1 = gam + (size_t)clip * nparts * nb2 + (size_t)(a + g.Ny) * g.nbx + (b + g.Nx);
     const float2* p2 = gam + (size_t)clip * nparts * nb2 + (size_t)(g.Ny - a) * g.nbx + (g.Nx - b);
-#pragma unroll 8
+#pragma unroll 16
     for (int p = 0; p < nparts; ++p) {
       f1 = cadd(f1, __ldg(p1 + p * nb2));
       f2 = cadd(f2, __ldg(p2 + p * nb2));
