@@ -142,9 +142,10 @@ int kl_socs_plan_engine(kl_socs_plan plan);
  * image error of the same order as the CUDA-core engine's; mask values within
  * +-2^15, others are reported by kl_socs_plan_status); KL_SYNTH_AUTO
  * (the default), the engine kl_socs_autotune picked, else the CUDA cores.
- * kl_socs_vjp runs its image, resist and gradient syntheses on the tensor
- * cores wherever the geometry allows, unless KL_SYNTH_CUDA_CORES is set, and
- * its mask transform there only with KL_SYNTH_TENSOR_CORES.
+ * kl_socs_vjp with KL_SYNTH_AUTO runs its image, resist and gradient syntheses
+ * on the tensor cores wherever the geometry allows and the call has more than
+ * 64 x 128 image rows (clips x kernel sets x Ly), and its mask transform there
+ * only with KL_SYNTH_TENSOR_CORES.
  * Returns KL_ERR_UNSUPPORTED for the tensor-core engine on other geometries
  * and on general-pipeline plans.  No counterpart in the reference. */
 #define KL_SYNTH_AUTO 0

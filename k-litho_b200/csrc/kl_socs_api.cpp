@@ -471,9 +471,14 @@ int kl_socs_vjp(kl_socs_plan p, const float* masks, const float* targets, int nc
   if (rc) return rc;
   if ((rc = spectral(p, nclips, kl::spec_choose_split(p->sg, nclips * p->nsets, p->K), st))) return rc;
   KL_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(double) * (size_t)nclips * p->nsets, st));
-  // image, resist, loss and the row DFT of dL/dI: on the tensor cores where
-  // the plan has them, unless it asks for the CUDA-core engine
-  const bool tca = p->vjp_tc && p->synth != KL_SYNTH_CUDA_CORES &&
+  // image, resist, loss and the row DFT of dL/dI, and the gradient's synthesis: on the
+  // tensor cores where the plan has them, unless it asks for the CUDA-core engine.  Their
+  // kernels have a CTA per one or two tiles of 128 rows, the CUDA cores' one per 32 rows:
+  // up to 64 image tiles those are faster, us a call of 1, 8, 12 and 32 clips (tensor
+  // cores first): 512^2 99 / 74, 96 / 74, 100 / 86 (48 tiles), 107 / 117; 1024^2 160 / 131,
+  // 163 / 137 (64 tiles), 172 / 166, 254 / 260; 768^2 141 / 141, 143 / 145, 145 / 156, 211 / 266
+  const bool few = p->synth == KL_SYNTH_AUTO && (size_t)nclips * p->nsets * g.Ly <= 64 * 128;
+  const bool tca = p->vjp_tc && p->synth != KL_SYNTH_CUDA_CORES && !few &&
                    (((uintptr_t)targets | (uintptr_t)images) & 15) == 0;
   rc = tca ? kl::vjp_tc_launch(g, p->T, p->ty, nclips, p->nsets, p->bhi, p->blo, p->thi, p->tlo, targets, alpha,
                                threshold, images, loss, p->gpart, p->status, st)
@@ -487,9 +492,8 @@ int kl_socs_vjp(kl_socs_plan p, const float* masks, const float* targets, int nc
   if ((rc = kl::adjoint_gradient(p->sg, p->gam, nclips, p->nsets * adjoint_parts(p, ns2), 2 * g.Ny, g.ntx, g.ntx, 1, p->Tg,
                                  st)))
     return rc;
-  // the gradient is a band-limited synthesis like the image: on the tensor
-  // cores unless the plan asks for the CUDA-core engine
-  const bool tcg = p->bhi && p->synth != KL_SYNTH_CUDA_CORES && kl::synth_tc_aligned(grad);
+  // the gradient is a band-limited synthesis like the image
+  const bool tcg = p->bhi && p->synth != KL_SYNTH_CUDA_CORES && !few && kl::synth_tc_aligned(grad);
   rc = tcg ? kl::synth_tc_launch(g, p->Tg, p->ty, p->bhi, p->blo, nclips, grad, p->status, st)
            : kl::socs_launch_inverse(g, p->tx, p->ty, p->Tg, nclips, 1, grad, st);
   if (rc) return rc;
