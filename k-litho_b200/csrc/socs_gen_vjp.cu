@@ -527,8 +527,9 @@ int launch_rowvjp_t(const GenGeom& g, const float2* tables, float2* Q, int nimg,
     if (fold) kern = k_gen_rowvjp<PF, true>;
   int rc = set_smem(kern, sm);
   if (rc) return rc;
-  // about four CTAs per SM over the whole batch, each on rows of one image
-  int bx = (4 * kSMs + nimg - 1) / nimg;
+  // about two CTAs per SM over the whole batch, as many as fit, each on rows of one image:
+  // four 2048^2 clips 227 us a call, 238, 230 and 231 with three, four and six per SM
+  int bx = (2 * kSMs + nimg - 1) / nimg;
   bx = std::max(1, std::min(bx, (g.Ly + kW - 1) / kW));
   kern<<<dim3(bx, nimg), kT, sm, st>>>(Q, g, tables, gen_roots_x(g, tables), nsets, targets, alpha, thr,
                                           images, loss);
