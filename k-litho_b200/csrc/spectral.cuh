@@ -141,6 +141,8 @@ __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
   const int img = blockIdx.x / CL, c0 = (blockIdx.x - img * CL) * RC, split = blockIdx.y;
   const int clip = img / nsets, set = img - clip * nsets;
   const int k0 = (int)(((long long)K * split) / nsplit), k1 = (int)(((long long)K * (split + 1)) / nsplit);
+  // last kernel first: kernels come sorted by weight, so the sums stay small until the end
+  // (64 kernels at 4096^2: error against 64 bits 3.6e-7 in order, 2.9e-7 in reverse)
   const int nbatch = (k1 - k0 + KB - 1) / KB;
 
   // row role: kernel slot, x residue and band row
@@ -155,13 +157,13 @@ __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
   if (rowthr) {
     hleft = (k1 - k0 - slot1 + KB - 1) / KB;
     if (hleft > 0) {
-      hk = H + ((size_t)set * K + k0 + slot1) * hs + (NATURAL ? (size_t)row1 * g.nbx + g.Nx : row1);
+      hk = H + ((size_t)set * K + (k1 - 1 - slot1)) * hs + (NATURAL ? (size_t)row1 * g.nbx + g.Nx : row1);
       h0 = __ldg(hk);
     }
     if constexpr (!NATURAL) {
       feed.h = hleft > 0 ? hk + spec_n0(g) + row1 : H;
       feed.pair = 2 * nby;
-      feed.skip = (ptrdiff_t)((KB - 1) * hs) + spec_n0(g);
+      feed.skip = spec_n0(g) - (ptrdiff_t)((KB + 1) * hs);
       feed.ring = (unsigned)__cvta_generic_to_shared(sm + L.ring + 2 * tid);
       feed.q = feed.put = 0;
       feed.left = hleft;
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
         if constexpr (RG == 1) static_for<9, 24>([&](auto j) { v[j] = make_float2(0.f, 0.f); });
         // the next batch's value at n = 0
         if (--hleft > 0) {
-          hk += (size_t)KB * hs;
+          hk -= (size_t)KB * hs;
           h0 = __ldg(hk);
         } else {
           h0 = make_float2(0.f, 0.f);
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
       float2 v[32];
       if (b < nbatch) {
         const int k2 = b * KB + slot2;
-        if (k2 < k1 - k0) lk = __ldg(lams + k2);
+        if (k2 < k1 - k0) lk = __ldg(lams + (k1 - k0 - 1 - k2));
         bar_sync<kT>(kFull + (b & 1));
         const float2* e = e1r + (b & 1) * kE1;
         if constexpr (RG <= 2) {
