@@ -16,12 +16,12 @@
 //            the register count does not grow with the band).
 //  col_fwd   the row bins' DFT along y, kept for |fy| <= Ny: 32-point warp FFTs
 //            over strips of 32 rows spaced Ly/32 apart when 32 divides Ly,
-//            otherwise a direct sum; strips are split over `nparts` partial bands.
+//            otherwise blocks of 32 rows by one table; strips are split over `nparts` partial bands.
 //  spectral  (spectral.cu) the band's K fields, their lambda |E|^2 and its
 //            spectrum T, on chip.
-//  col_inv   T's columns synthesised along y for every image row (strip FFTs
-//            or a direct sum), giving the rows' coefficients Q[y][b], b <= 2Nx.
-//  row_inv   (HBM-bound) each warp synthesises image rows from Q: lane l'
+//  col_inv   T's columns synthesised along y for every image row (a strip's
+//            32-point FFT per thread, or the blocks), giving the rows' coefficients Q[y][b], b <= 2Nx.
+//  row_inv   each warp synthesises image rows from Q: lane l'
 //            accumulates the Hermitian half of its P sub-bins and runs one
 //            length-P complex-to-real transform in registers.
 //

@@ -18,10 +18,9 @@
 //   dL/dJ_s = sum_x G(x) |E_s(x)|^2 = (1/G^2) sum_p gam(p) |e_s(p)|^2 / J_s
 // with e_s built from the kernel conj(A[:, s]).
 //
-// Kernels: k_vjp_inverse (image rows + loss + row DFT of G, fused; HBM-bound),
-// k_vjp_spectral (per clip and kernel slice: Gam), k_vjp_gradT (Gam -> the
-// half-plane spectrum of the gradient, synthesised by k_socs_inverse), and
-// k_vjp_source (per clip and source slice: dL/dJ).
+// Kernels: k_vjp_inverse (image rows + loss + row DFT of G, fused) and k_vjp_source
+// (per clip and source slice: dL/dJ); Gam and the half-plane spectrum of the
+// gradient come from adjoint_spectral.cu, its synthesis from k_socs_inverse.
 #include <cuda_pipeline.h>
 
 #include <algorithm>

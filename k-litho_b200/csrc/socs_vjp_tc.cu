@@ -16,7 +16,7 @@
 //      basis (same 3-term FP16 split), over the tile's 64-column blocks;
 //   4. at the end of the tile the epilogue warps read Gr, run the J-point
 //      column FFTs of each strip and write its partial band spectrum of G
-//      (|gy| <= 2Ny, the layout k_vjp_spectral reads), exactly as
+//      (|gy| <= 2Ny, the layout k_adjoint_gamma reads), exactly as
 //      k_vjp_inverse does on the CUDA cores.
 // The model is the adjoint of K-Litho-SOCS/klitho_socs.cpp:158-241 (calcSOCS +
 // FI) under the sigmoid resist at the reference's TARGET_INTENSITY
