@@ -60,7 +60,7 @@ struct AdjSmem {
 // band, so the loads in flight bound it: four images at G = 128 (16 bands of 96 KB each)
 // 33 us with 16 float2 per thread, 23 with 32.
 template <int RG>
-__global__ void __launch_bounds__(512) k_adjoint_gamma(const float2* __restrict__ gband, int gparts, const SpecGeom g,
+__global__ void __launch_bounds__(512) k_adjoint_gamma(const float2* gband, int gparts, const SpecGeom g,
                                                        float* __restrict__ gamma) {
   constexpr int G = 32 * RG, kT = 512, kAhead = 16, kEach = 2;
   extern __shared__ float4 smem4[];
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(512) k_adjoint_gamma(const float2* __restrict_
       for (int e = 0; e < kEach; ++e)
 #pragma unroll
         for (int p = 0; p < kAhead; ++p)
-          x[e][p] = q0 + p < gparts && i0 + e * kT < per ? __ldg(p0 + (size_t)(q0 + p) * per + i0 + e * kT)
+          x[e][p] = q0 + p < gparts && i0 + e * kT < per ? p0[(size_t)(q0 + p) * per + i0 + e * kT]
                                                          : make_float2(0.f, 0.f);
 #pragma unroll
       for (int e = 0; e < kEach; ++e)
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(512) k_adjoint_gamma(const float2* __restrict_
 
 template <int RG>
 __global__ void __launch_bounds__(128, 2)
-    k_adjoint_spectral(const float2* __restrict__ band, int nparts, float scale, const float* __restrict__ gamma,
+    k_adjoint_spectral(const float2* band, int nparts, float scale, const float* gamma,
                        const SpecGeom g, const float2* __restrict__ H, const float* __restrict__ lam, int K,
                        int nsets, int nsplit, float2* __restrict__ gam_out) {
   using C = AdjCfg<RG>;
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(128, 2)
         float2 x[kAhead];
 #pragma unroll
         for (int p = 0; p < kAhead; ++p)
-          x[p] = p0 + p < nparts ? __ldg(b0 + (size_t)(p0 + p) * per + i) : make_float2(0.f, 0.f);
+          x[p] = p0 + p < nparts ? b0[(size_t)(p0 + p) * per + i] : make_float2(0.f, 0.f);
 #pragma unroll
         for (int p = 0; p < kAhead; ++p) v = cadd(v, x[p]);
       }
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(128, 2)
   if (warp < C::CW) {
     const float* gm = gamma + ((size_t)(img * RG + c0 + cc2) * RG + r2) * 1024 + lane;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) gam[i] = __ldg(gm + 32 * i);
+    for (int i = 0; i < 32; ++i) gam[i] = gm[32 * i];
   } else {
 #pragma unroll
     for (int i = 0; i < 32; ++i) gam[i] = 0.f;
@@ -412,7 +412,7 @@ int launch_adjoint(const SpecGeom& g, const float2* band, int nparts, float scal
 // T(a, b) = (conj Gam[a][b] + Gam[-a][-b]) / (Lx Ly) for |a| <= Ny, 0 <= b <= Nx, zero in
 // the rest of [-ay, ay] x [0, nb): the half-plane spectrum of dL/dm.  32 loads in flight
 // per thread: 32 shares of four images 10 us (31 with 16)
-__global__ void __launch_bounds__(128) k_adjoint_grad(const float2* __restrict__ gam, const SpecGeom g, int nparts, int ay,
+__global__ void __launch_bounds__(128) k_adjoint_grad(const float2* gam, const SpecGeom g, int nparts, int ay,
                                                       int nb, int sa, int sb, float2* __restrict__ T) {
   dep_wait();
   dep_launch();
@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(128) k_adjoint_grad(const float2* __restrict__
     const float2* p2 = gam + (size_t)clip * nparts * nb2 + (size_t)(g.Ny - a) * g.nbx + (g.Nx - b);
 #pragma unroll 16
     for (int p = 0; p < nparts; ++p) {
-      f1 = cadd(f1, __ldg(p1 + p * nb2));
-      f2 = cadd(f2, __ldg(p2 + p * nb2));
+      f1 = cadd(f1, p1[p * nb2]);
+      f2 = cadd(f2, p2[p * nb2]);
     }
   }
   T[(size_t)clip * rows * nb + (size_t)(a + ay) * sa + (size_t)b * sb] =

@@ -268,11 +268,11 @@ __device__ __forceinline__ void gen_load_hrow(const float2* __restrict__ Hk, int
 
 // Coefficients b = lane + 32 t (t < 4, b < nbins <= 128) of one row of a
 // row-coefficient array, as independent loads.
-__device__ __forceinline__ void gen_load_qrow(const float2* __restrict__ qr, int nbins, int lane, float2 (&q)[4]) {
+__device__ __forceinline__ void gen_load_qrow(const float2* qr, int nbins, int lane, float2 (&q)[4]) {
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     const int b = lane + 32 * t;
-    q[t] = b < nbins ? __ldg(qr + b) : make_float2(0.f, 0.f);
+    q[t] = b < nbins ? qr[b] : make_float2(0.f, 0.f);
   }
 }
 

@@ -7,6 +7,12 @@
 // Kernels call it before their first such access, and dep_launch() after it, so
 // at most one kernel is ahead.  Of a 25 us call on one 512^2 clip the launch gaps
 // are 4-5 us.
+//
+// Such a kernel is resident while its input is still being written.  So that input is
+// read by coherent loads that stay behind dep_wait(): plain ones through pointers
+// without __restrict__, or __ldcs and __ldcg (volatile).  __ldg and const __restrict__
+// promise data that nobody writes while the kernel runs, and such loads may be moved
+// above the wait; they are for the plan's tables and kernels only.
 #pragma once
 
 #include <cuda_runtime.h>

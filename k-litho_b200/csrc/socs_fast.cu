@@ -149,7 +149,7 @@ int socs_build_tables(const SocsGeom& g, float2* tx, float2* ty, cudaStream_t st
 // 1. forward: mask rows -> per-strip partial band spectra
 // ---------------------------------------------------------------------------
 template <int P, int V, int NFM, int RJ, int NT>
-__global__ void __launch_bounds__(NT) k_socs_forward(const float* __restrict__ masks,
+__global__ void __launch_bounds__(NT) k_socs_forward(const float* masks,
                                                            const SocsGeom g,
                                                            const float2* __restrict__ tx,
                                                            const float2* __restrict__ ty,
@@ -237,7 +237,7 @@ __device__ __forceinline__ void load_band(const float2* __restrict__ partial, co
 // 3. inverse: intensity spectrum -> image rows
 // ---------------------------------------------------------------------------
 template <int P, int V, int NBM, int RJ, int NT>
-__global__ void __launch_bounds__(NT) k_socs_inverse(const float2* __restrict__ T,
+__global__ void __launch_bounds__(NT) k_socs_inverse(const float2* T,
                                                            const SocsGeom g,
                                                            const float2* __restrict__ tx,
                                                            const float2* __restrict__ ty,
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(NT) k_socs_inverse(const float2* __restrict__ 
   dep_wait();
   dep_launch();
 #pragma unroll 4
-  for (int i = threadIdx.x; i < (int)tsz; i += NT) Ts[i] = __ldg(Ti + i);
+  for (int i = threadIdx.x; i < (int)tsz; i += NT) Ts[i] = Ti[i];
   float2 ph_next = make_float2(0.f, 0.f);
   if (threadIdx.x < g.nty) ph_next = __ldg(ty + (size_t)s0 * g.nty + threadIdx.x);
   __syncthreads();

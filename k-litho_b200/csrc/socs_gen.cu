@@ -215,7 +215,7 @@ int gen_build_tables(const GenGeom& g, float2* tables, cudaStream_t st) {
 // 1. row_fwd: rows of `src` (Lx floats each) -> R[row][fx], fx < nbins
 // ---------------------------------------------------------------------------
 template <int PF>
-__global__ void __launch_bounds__(kT) k_gen_rowfwd(const float* __restrict__ src, int nrows, const GenGeom g,
+__global__ void __launch_bounds__(kT) k_gen_rowfwd(const float* src, int nrows, const GenGeom g,
                                                    const float2* __restrict__ tables, int nbins,
                                                    float2* __restrict__ R) {
   constexpr int HS = PF / 2 + 1;
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kT) k_gen_rowfwd(const float* __restrict__ src
 // 2. col_fwd: R[n][y][fx] -> band[n][part][fy + Yb][fx], |fy| <= Yb, times scale;
 // periods of strips (Ly a multiple of 32)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R, int ncols, int Yb,
+__global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* R, int ncols, int Yb,
                                                    const GenGeom g, const float2* __restrict__ rly,
                                                    float scale, float2* __restrict__ band) {
   constexpr int MT = 8;  // 2 Yb + 1 <= 256
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R,
   // the next strip's row bin and phases are loaded while this strip is transformed
   float2 rn = make_float2(0.f, 0.f), pn[MT];
   auto fetch = [&](int s) {
-    rn = __ldg(Rn + (size_t)(s + nS * lane) * ncols + fx);
+    rn = Rn[(size_t)(s + nS * lane) * ncols + fx];
 #pragma unroll
     for (int t = 0; t < MT; ++t) {
       const int fy = fy0 + 32 * t;
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd(const float2* __restrict__ R,
 // (the same 32 x 64 table for every block) and turns the block's sum by
 // e^{-2 pi i fy 32 s/Ly}.  Thread = one column fx, four fy.  One frequency per lane with
 // both factors gathered for every row took 102 us for seven 1000 x 744 clips.
-__global__ void __launch_bounds__(kT) k_gen_colfwd_blocks(const float2* __restrict__ R, int ncols, int Yb,
+__global__ void __launch_bounds__(kT) k_gen_colfwd_blocks(const float2* R, int ncols, int Yb,
                                                           const GenGeom g, const float2* __restrict__ rly, int nparts,
                                                           float scale, float2* __restrict__ band) {
   __shared__ float2 Rt[32][16];
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd_blocks(const float2* __restri
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int y = 32 * s + ty + 16 * h;
-      next[h] = colok && y < Ly ? __ldg(Rn + (size_t)y * ncols) : make_float2(0.f, 0.f);
+      next[h] = colok && y < Ly ? Rn[(size_t)y * ncols] : make_float2(0.f, 0.f);
     }
   };
   float2 acc[4];
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kT) k_gen_colfwd_blocks(const float2* __restri
 // 49 us; 117 with one transform spread over a warp's lanes by shuffles.
 __host__ __device__ inline int colinv_rows(int A) { return (A + 7) / 8 * 8 + (A + 8) / 8 * 8; }
 
-__global__ void __launch_bounds__(kT, 2) k_gen_colinv(const float2* __restrict__ T, int A, int nbins,
+__global__ void __launch_bounds__(kT, 2) k_gen_colinv(const float2* T, int A, int nbins,
                                                       const GenGeom g, const float2* __restrict__ rly,
                                                       float2* __restrict__ Q, int spw) {
   extern __shared__ float4 smem4[];
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kT, 2) k_gen_colinv(const float2* __restrict__
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
       const int i = alo + A + lane + 32 * t;
-      x[t] = i >= 0 && i < lda && b < nbins ? __ldg(Ti + (size_t)b * lda + i) : make_float2(0.f, 0.f);
+      x[t] = i >= 0 && i < lda && b < nbins ? Ti[(size_t)b * lda + i] : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int t = 0; t < 8; ++t)
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kT, 2) k_gen_colinv(const float2* __restrict__
 // (MB of them) of SB blocks: one table value serves all.  A row per lane with both
 // factors gathered for every term took 20 us for 14 images of 1000 x 744.
 template <int MB, int SB>
-__global__ void __launch_bounds__(kT) k_gen_colinv_blocks(const float2* __restrict__ T, int A, int nbins,
+__global__ void __launch_bounds__(kT) k_gen_colinv_blocks(const float2* T, int A, int nbins,
                                                           const GenGeom g, const float2* __restrict__ rly,
                                                           float2* __restrict__ Q) {
   extern __shared__ float4 smem4[];
@@ -531,7 +531,7 @@ __global__ void __launch_bounds__(kT) k_gen_colinv_blocks(const float2* __restri
 #pragma unroll
     for (int q = 0; q < MB; ++q) {
       const int b = warp + kW * q;
-      const float2 t = a < lda && b < nbins ? __ldg(Ti + (size_t)b * lda + a) : make_float2(0.f, 0.f);
+      const float2 t = a < lda && b < nbins ? Ti[(size_t)b * lda + a] : make_float2(0.f, 0.f);
 #pragma unroll
       for (int s = 0; s < SB; ++s) Tt[(size_t)(s * 32 + lane) * NB + b] = cmul(t, ph[s]);
     }
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kT) k_gen_colinv_blocks(const float2* __restri
 // 4. row_inv: Q[row][b] (b < nbins) -> out[row][x] = Re sum_b Q[b] e^{2 pi i b x/Lx}
 // ---------------------------------------------------------------------------
 template <int P>
-__global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* __restrict__ Q, int nbins, int nrows,
+__global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* Q, int nbins, int nrows,
                                                    const GenGeom g, const float2* __restrict__ tables,
                                                    float* __restrict__ out) {
   constexpr int HY = P / 2 + 1;
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* __restrict__ Q,
 
 // The same for P >= 8 with the twiddles factored (row_fold.cuh).
 template <int P, bool SM>
-__global__ void __launch_bounds__(kT) k_gen_rowinv_fold(const float2* __restrict__ Q, int nbins, int nrows,
+__global__ void __launch_bounds__(kT) k_gen_rowinv_fold(const float2* Q, int nbins, int nrows,
                                                         const GenGeom g, const float2* __restrict__ rlx,
                                                         float* __restrict__ out) {
   extern __shared__ float4 smem4[];

@@ -37,7 +37,7 @@ int set_smem(Kern k, size_t bytes) {
 // out[row][x] = Re sum_b Q[row][b] e^{2 pi i b x/Lx}.  A CTA keeps the twiddles of its 64
 // pixels and walks over tiles of 64 rows; a warp has 8 rows x 2 pixels per lane, and
 // their mirrors: 64 FMAs per 12 shared loads.
-__global__ void __launch_bounds__(kT) k_row_synth(const float2* __restrict__ Q, int nbins, int nrows, int Lx,
+__global__ void __launch_bounds__(kT) k_row_synth(const float2* Q, int nbins, int nrows, int Lx,
                                                   const float2* __restrict__ rlx, float* __restrict__ out) {
   extern __shared__ float4 smem4[];
   const int nbp = (nbins + 1) & ~1;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kT) k_row_synth(const float2* __restrict__ Q, 
     __syncthreads();
     for (int i = tid; i < kRows * nbins; i += kT) {
       const int r = i / nbins, b = i - r * nbins;
-      qs[(size_t)r * nbp + b] = r < nr ? __ldg(Q + (size_t)r0 * nbins + i) : make_float2(0.f, 0.f);
+      qs[(size_t)r * nbp + b] = r < nr ? Q[(size_t)r0 * nbins + i] : make_float2(0.f, 0.f);
     }
     __syncthreads();
     float C[8][2], S[8][2];
@@ -109,8 +109,8 @@ __global__ void __launch_bounds__(kT) k_row_synth(const float2* __restrict__ Q, 
 // VJP: m is dL/dI of the sigmoid resist, made from the image and its target on the
 // way; the loss is added to loss[image].
 template <int F, int RPT, bool VJP>
-__global__ void __launch_bounds__(kT) k_row_dft(const float* __restrict__ src, int Ly, int Lx, int nbins,
-                                                const float2* __restrict__ rlx, const float* __restrict__ targets,
+__global__ void __launch_bounds__(kT) k_row_dft(const float* src, int Ly, int Lx, int nbins,
+                                                const float2* __restrict__ rlx, const float* targets,
                                                 int nsets, float alpha, float thr, double* __restrict__ loss,
                                                 float2* __restrict__ R) {
   constexpr int ROWS = 16 * RPT, UP = ROWS + 2, LD = ROWS / kW;  // row pairs (u, v) loaded per thread
@@ -139,9 +139,9 @@ __global__ void __launch_bounds__(kT) k_row_dft(const float* __restrict__ src, i
     for (int k = 0; k < LD; ++k) {
       const int r = warp + kW * k;
       const bool ok = x <= half && r0 + r < Ly, mir = ok && x > 0 && 2 * x != Lx;
-      a[k] = make_float2(ok ? __ldg(m + (size_t)r * Lx + x) : 0.f, mir ? __ldg(m + (size_t)r * Lx + Lx - x) : 0.f);
+      a[k] = make_float2(ok ? m[(size_t)r * Lx + x] : 0.f, mir ? m[(size_t)r * Lx + Lx - x] : 0.f);
       if constexpr (VJP)
-        t[k] = make_float2(ok ? __ldg(tg + (size_t)r * Lx + x) : 0.f, mir ? __ldg(tg + (size_t)r * Lx + Lx - x) : 0.f);
+        t[k] = make_float2(ok ? tg[(size_t)r * Lx + x] : 0.f, mir ? tg[(size_t)r * Lx + Lx - x] : 0.f);
     }
   };
   float2 acc[RPT][F];

@@ -107,7 +107,7 @@ __global__ void k_synth_basis(int Lx, int ntx, int Kp, __half* __restrict__ bhi,
 
 template <int RJ, int KA>
 __global__ void __launch_bounds__(kSThreads, 1)
-    k_socs_synth_tc(const float2* __restrict__ T, const SocsGeom g, const float2* __restrict__ ty,
+    k_socs_synth_tc(const float2* T, const SocsGeom g, const float2* __restrict__ ty,
                     const __grid_constant__ CUtensorMap tm_hi, const __grid_constant__ CUtensorMap tm_lo,
                     const __grid_constant__ CUtensorMap tm_img, int nimg, int* __restrict__ err) {
   constexpr int J = 32 * RJ;
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kSThreads, 1)
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             const int i = i0 + u * 32 * kCW, ar = i / tstr, b = i - ar * tstr;
-            v[u] = (i < nty * tstr && b < ntx) ? __ldg(Ti + (size_t)ar * ntx + b) : make_float2(0.f, 0.f);
+            v[u] = (i < nty * tstr && b < ntx) ? Ti[(size_t)ar * ntx + b] : make_float2(0.f, 0.f);
           }
 #pragma unroll
           for (int u = 0; u < 8; ++u) {

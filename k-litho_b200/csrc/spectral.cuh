@@ -119,7 +119,7 @@ __device__ __forceinline__ void put_T(const SpecGeom& g, float2* __restrict__ T,
 // larger grids [image][slice][x residue][4Ny+1][32] sums over the y residues.
 template <int RG, bool NATURAL>
 __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
-    k_spectral(const float2* __restrict__ band, int nparts, float scale, const SpecGeom g,
+    k_spectral(const float2* band, int nparts, float scale, const SpecGeom g,
                const float2* __restrict__ H, const float* __restrict__ lam, int K, int nsets, int nsplit,
                float2* __restrict__ part, float2* __restrict__ T, unsigned* __restrict__ done) {
   using C = SpecCfg<RG>;
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
       float2 x[kAhead];
 #pragma unroll
       for (int p = 0; p < kAhead; ++p)
-        x[p] = p0 + p < nparts ? __ldg(b0 + (size_t)(p0 + p) * per + i) : make_float2(0.f, 0.f);
+        x[p] = p0 + p < nparts ? b0[(size_t)(p0 + p) * per + i] : make_float2(0.f, 0.f);
 #pragma unroll
       for (int p = 0; p < kAhead; ++p) v = cadd(v, x[p]);
     }
@@ -442,7 +442,7 @@ __global__ void __launch_bounds__(SpecCfg<RG>::T, 1)
 // T(a, b) of each image: its slices' spectra added up (up to 64 points), or
 // sum_c w_G^{-b c} of the slices' x residues
 template <int RG>
-__global__ void __launch_bounds__(256) k_spec_sum(const float2* __restrict__ part, const SpecGeom g, int nsplit,
+__global__ void __launch_bounds__(256) k_spec_sum(const float2* part, const SpecGeom g, int nsplit,
                                                   float2* __restrict__ T) {
   constexpr int G = 32 * RG;
   const int tsz = g.nty * g.ntx, i = blockIdx.y * 256 + threadIdx.x, img = blockIdx.x;
