@@ -22,6 +22,23 @@ int scratch_alloc(void** p, size_t bytes, cudaStream_t st, const char* what);
 void scratch_free(void* p, cudaStream_t st);
 const char* last_error();
 
+// The current device for a scope, the caller's again after it.  Calls that only copy
+// find a plan's device by the address; what they launch or allocate must be told.
+struct OnDevice {
+  int before = -1;
+  cudaError_t status;
+  explicit OnDevice(int device) {
+    status = cudaGetDevice(&before);
+    if (status == cudaSuccess && before != device) status = cudaSetDevice(device);
+    else before = -1;
+  }
+  ~OnDevice() {
+    if (before >= 0) cudaSetDevice(before);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+};
+
 #define KL_CUDA_TRY(expr)                                                      \
   do {                                                                         \
     cudaError_t _e = (expr);                                                   \

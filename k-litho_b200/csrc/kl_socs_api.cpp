@@ -395,8 +395,11 @@ namespace {
 // kernels of one set from the host, interleaved (im null) or as two planes: copied as
 // they are and put in order on the device -- interleaving 6 MB on the host took
 // longer than the copy.  The kernel layout is kept where an adjoint needs it,
-// else only on the way to the spectral core's.  Done on return.
+// else only on the way to the spectral core's.  On the plan's device, whichever is
+// current.  Done on return.
 int upload_kernels(kl_socs_plan p, int set, const float* re, const float* im, const float* scales) {
+  const kl::OnDevice on(p->device);
+  KL_CUDA_TRY(on.status);
   const size_t n = (size_t)p->g.nby * p->g.nbx * p->K, k0 = (size_t)set * p->K;
   void* tmp = nullptr;
   const size_t tmp_floats = (p->H ? 0 : 2 * n) + (im ? 2 * n : 0);
