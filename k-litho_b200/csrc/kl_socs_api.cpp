@@ -362,9 +362,12 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
   if ((rc = kl::gen_launch_colinv(g, p->gtab, p->T, nimg, 2 * g.Ny, g.ntx, p->Q, st))) return rc;
   KL_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(double) * (size_t)nimg, st));
   // image, then dL/dI's row bins from it; without a place for the image (no output
-  // for it, several images per clip) both in one kernel.  The gradient is written last
+  // for it, several images per clip, an output over the targets, which are still to be
+  // read) both in one kernel.  The gradient is written last
   float* im = images ? images : p->nsets == 1 ? grad : nullptr;
-  if (kl::gen_direct_dft(g) && im) {
+  const size_t px = (size_t)g.Lx * g.Ly;
+  const bool over = im && im < targets + px * nclips && targets < im + px * nimg;
+  if (kl::gen_direct_dft(g) && im && !over) {
     const float2* rlx = kl::gen_roots_x(g, p->gtab);
     if ((rc = kl::row_synth(g, rlx, p->Q, nimg * g.Ly, g.ntx, im, st))) return rc;
     rc = kl::row_dft_vjp(g, rlx, im, nimg, g.ntx, targets, p->nsets, alpha, threshold, loss, p->Q, st);
