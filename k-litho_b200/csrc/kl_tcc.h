@@ -93,7 +93,8 @@ struct FactorProblem {
 // Top-K eigenpairs of several TCC = A A^H at once (e.g. one per focus value):
 // factors with S <= 256 columns share one batched Gram eigensolve; the rest
 // are solved one after another by subspace iteration.
-// `meanwhile` (may be empty) is host work done once while the GPU solves.
+// `meanwhile` (may be empty) is host work done once while the GPU solves in one step
+// (S <= 256); the iteration, whose checks keep the host busy, leaves it out.
 int eig_topk_factor_batch(const std::vector<FactorProblem>& problems, const EigenOptions& opt,
                           cudaStream_t st, const std::function<void()>& meanwhile);
 

@@ -273,11 +273,16 @@ struct TopkBuffers {
 
 // Writes one byte of every page of an output that will be overwritten: fresh host
 // memory (29 MB for 64 kernels of a 4096^2 field at five focus values) gets its
-// pages while the GPU solves instead of during the copy.
+// pages while the GPU solves instead of during the copy.  The byte keeps its value: a
+// solve that fails leaves the caller's arrays as they were.
 void touch_pages(void* p, size_t bytes) {
   volatile char* c = static_cast<volatile char*>(p);
-  for (size_t i = 0; i < bytes; i += 4096) c[i] = 0;
-  if (bytes) c[bytes - 1] = 0;
+  auto touch = [&](size_t i) {
+    const char v = c[i];
+    c[i] = v;
+  };
+  for (size_t i = 0; i < bytes; i += 4096) touch(i);
+  if (bytes) touch(bytes - 1);
 }
 
 kl::EigenOptions topk_options(int K, int block) {
