@@ -188,13 +188,15 @@ int kl_socs_forward_host(kl_socs_plan plan, const float* masks_host, int nclips,
 /* ------------------------------------------------------------------------- */
 
 /* Times the plan's launch shapes for batches of nclips clips (kernel slices of
- * the spectral stage: 1, 2, 4, 8; image strips per CTA of the synthesis stage:
- * 1 .. 16; the tensor-core synthesis where the geometry allows it) with CUDA
- * events on `stream` and keeps the fastest; later calls of kl_socs_forward
- * with nclips clips use it.  Writes images_dev (the images of the chosen
- * shape).  Synchronous.  The chosen shape is returned in *nsplit / *spc when
- * those are not NULL (*spc = -1: the tensor-core synthesis, -2: the tensor-core
- * synthesis and mask transform). */
+ * the spectral stage: 1, 2, 4, 8 and the untuned plan's count; image strips
+ * per CTA of the synthesis stage: 1 .. 16; the tensor-core synthesis where the
+ * geometry allows it) with CUDA events on `stream` and keeps the fastest;
+ * later calls of kl_socs_forward with nclips clips use it.  Writes images_dev
+ * (the images of the chosen shape).  Synchronous.  *nsplit, when not NULL,
+ * receives the fastest of 1, 2, 4 and 8 slices, also where the plan stays with
+ * its untuned count because that is faster still; *spc the strips per CTA (-1:
+ * the tensor-core synthesis, -2: the tensor-core synthesis and mask
+ * transform). */
 int kl_socs_autotune(kl_socs_plan plan, const float* masks_dev, int nclips, float* images_dev,
                      void* stream, int* nsplit, int* spc);
 

@@ -84,9 +84,12 @@ int kl_socs_autotune(kl_socs_plan p, const float* masks, int nclips, float* imag
   cudaStream_t st = (cudaStream_t)stream;
   const bool timing = p->timing;
   p->timing = false;
-  std::vector<int> splits, spcs;
+  // beside 1, 2, 4 and 8 the untuned plan's count (any up to 64; the plan's sums hold
+  // it), so that a tuned plan is no slower
+  const int nimg = nclips * p->nsets, untuned = kl::spec_choose_split(p->sg, nimg, p->K);
+  std::vector<int> splits{untuned}, spcs;
   for (int ns : {1, 2, 4, 8})
-    if (ns <= p->K && kl::spec_part_elems(p->sg, nclips * p->nsets, ns) <= p->part_cap) splits.push_back(ns);
+    if (ns != untuned && ns <= p->K && kl::spec_part_elems(p->sg, nimg, ns) <= p->part_cap) splits.push_back(ns);
   // strips per CTA of the synthesis: specialised kernels only
   if (!p->gen)
     for (int c = 1; c <= 16 && c <= p->g.nS; c *= 2) spcs.push_back(c);
@@ -108,14 +111,18 @@ int kl_socs_autotune(kl_socs_plan p, const float* masks, int nclips, float* imag
     KL_CUDA_TRY(cudaEventElapsedTime(ms, e0, e1));
     return KL_OK;
   };
-  int best_ns = splits.empty() ? 1 : splits[0], best_spc = 0;
-  float best = 1e30f, t = 0.f;
+  int best_ns = untuned, best_listed = 1, best_spc = 0;
+  float best = 1e30f, listed = 1e30f, t = 0.f;
   // kernel slices of the spectral stage, with the default inverse shape ...
   for (int ns : splits) {
     if ((rc = time_shape(ns, 0, &t))) break;
     if (t < best) {
       best = t;
       best_ns = ns;
+    }
+    if ((ns == 1 || ns == 2 || ns == 4 || ns == 8) && t < listed) {
+      listed = t;
+      best_listed = ns;
     }
   }
   // ... then strips per CTA of the inverse stage, and the tensor-core synthesis
@@ -143,7 +150,7 @@ int kl_socs_autotune(kl_socs_plan p, const float* masks, int nclips, float* imag
   p->tune_spc = best_spc;
   // leave the images of the chosen shape in the output
   if ((rc = kl::socs_run_forward(p, masks, nclips, images, st, nullptr))) return rc;
-  if (nsplit_out) *nsplit_out = best_ns;
+  if (nsplit_out) *nsplit_out = best_listed;
   if (spc_out) *spc_out = best_spc;
   return KL_OK;
 }

@@ -11,7 +11,8 @@ CSRC = os.path.join(REPO, "k-litho_b200", "csrc")
 HARNESS = os.path.join(REPO, "tests", "harness")
 
 
-@pytest.mark.parametrize("program,source", [("upload_device", "kl_socs_api.cpp"), ("topk_outputs", "kl_tcc_api.cpp")])
+@pytest.mark.parametrize("program,source", [("upload_device", "kl_socs_api.cpp"), ("topk_outputs", "kl_tcc_api.cpp"),
+                                            ("autotune_slices", "kl_socs_batch.cpp")])
 def test_host_path(tmp_path, program, source):
     exe = str(tmp_path / program)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
