@@ -8,6 +8,15 @@
 // at most one kernel is ahead.  Of a 25 us call on one 512^2 clip the launch gaps
 // are 4-5 us.
 //
+// A kernel that starts ahead gets the SMs its predecessor leaves free then, not an even
+// share: a mask transform of one or two CTAs per SM, started at the beginning of the
+// previous call's row synthesis, took twice as long.  So the general pipeline's row
+// syntheses, a call's last kernels, call dep_launch() when their rows are written.
+// Calls back to back, us, at the beginning and at the end: one 2004 x 1184 clip 77 / 40,
+// one 2008 x 2016 64 / 39, eight 1002 x 744 81 / 58, seven 1000 x 744 at two focus values
+// 94 / 86; where the transform fills the SMs the earlier start was 2 us better, eight
+// 2080 x 2048 119 / 122.
+//
 // Such a kernel is resident while its input is still being written.  So that input is
 // read by coherent loads that stay behind dep_wait(): plain ones through pointers
 // without __restrict__, or __ldcs and __ldcg (volatile).  __ldg and const __restrict__

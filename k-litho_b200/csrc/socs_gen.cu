@@ -584,7 +584,6 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* Q, int nbins, i
     for (int i = threadIdx.x; i < nch * g.NBX; i += kT) t2s[i] = __ldg(tables + off_tw2(g) + i);
   __syncthreads();
   dep_wait();
-  dep_launch();
   const int nbp = (nbins + P - 1) / P * P;
   // each lane holds the coefficients b = lane + 32 t of its warp's row; the
   // next row's are loaded while the current one is synthesised
@@ -633,6 +632,7 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv(const float2* Q, int nbins, i
       __syncwarp();
     }
   }
+  dep_launch();  // the next call's kernel, see kl_launch.cuh
 }
 
 // The same for P >= 8 with the twiddles factored (row_fold.cuh).
@@ -648,7 +648,6 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv_fold(const float2* Q, int nbi
   if (SM) row_fold_tables<P>(rlx, V, threadIdx.x, kT, tb);
   __syncthreads();
   dep_wait();
-  dep_launch();
   const int nbp = (nbins + P - 1) / P * P;
   float2 qn[4];
   const int row0 = blockIdx.x * kW + warp, rstep = gridDim.x * kW;
@@ -674,6 +673,7 @@ __global__ void __launch_bounds__(kT) k_gen_rowinv_fold(const float2* Q, int nbi
       }
     }
   }
+  dep_launch();  // as above
 }
 
 // centred FT_r2c band: M(ky,kx) = D(ky,kx) e^{-2 pi i (ky yh/Ly + kx xh/Lx)}

@@ -52,7 +52,6 @@ __global__ void __launch_bounds__(kT) k_row_synth(const float2* Q, int nbins, in
   if (nbp > nbins)
     for (int i = tid; i < kRows; i += kT) qs[(size_t)i * nbp + nbins] = make_float2(0.f, 0.f);
   dep_wait();
-  dep_launch();
   const int half = Lx / 2;
   for (int r0 = blockIdx.y * kRows; r0 < nrows; r0 += gridDim.y * kRows) {
     const int nr = min(kRows, nrows - r0);
@@ -100,6 +99,7 @@ __global__ void __launch_bounds__(kT) k_row_synth(const float2* Q, int nbins, in
       }
     }
   }
+  dep_launch();  // the next call's kernel, see kl_launch.cuh
 }
 
 // R[row][fx] = sum_x m[row][x] e^{-2 pi i fx x/Lx}, fx < nbins, of the rows of one image
