@@ -31,7 +31,13 @@ SpecGeom spec_geometry(const GenGeom& s) {
 
 int spec_choose_split(const SpecGeom& g, int nimg, int K) {
   // The slice count with the least waves x (batches of kernels + fixed part of a
-  // CTA, about three batches: band load, back transform, slice sum).
+  // CTA, about three batches: band load, back transform, slice sum).  At 32 points a CTA
+  // is small and several share an SM: waves count in fractions, of about 100 CTAs since
+  // the early start does not spread them evenly, and the sum over slices weighs as much
+  // as the fixed part.  With whole waves 12 to 48 kernels of 24 to 48 clips of 256^2 took
+  // up to 1.09 of the warp-FFT kernels' time; 32 clips of 24 kernels (3 slices, now 1)
+  // 28.3 -> 23.6 us a call.  Over 384 shapes 1.008 of the best count's time in the
+  // geometric mean (1.058 with whole waves).
   const int rg = g.G / 32, kb = rg == 1 ? 8 : rg <= 5 ? 2 : 1;
   const long long slots = 148, ctas = (long long)nimg * (rg == 2 ? 1 : rg);
   int best = 1;
@@ -39,8 +45,8 @@ int spec_choose_split(const SpecGeom& g, int nimg, int K) {
   const int most = std::min(kSpecMaxSplit, (K + kb - 1) / kb);
   for (int ns = 1; ns <= most; ++ns) {
     const int batches = ((K + ns - 1) / ns + kb - 1) / kb;
-    const long long waves = (ctas * ns + slots - 1) / slots;
-    const double t = (double)waves * (3.0 + batches) + 0.05 * ns;
+    const double waves = rg == 1 ? std::max(1.0, ctas * ns / 100.0) : (double)((ctas * ns + slots - 1) / slots);
+    const double t = waves * (3.0 + batches) + (rg > 1 ? 0.05 * ns : ns > 1 ? 3.0 + 0.4 * ns : 0.4);
     if (t < best_t * 0.98) {
       best_t = t;
       best = ns;
