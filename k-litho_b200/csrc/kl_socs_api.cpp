@@ -397,33 +397,53 @@ int vjp_gen(kl_socs_plan p, const float* masks, const float* targets, int nclips
 namespace {
 // kernels of one set from the host, interleaved (im null) or as two planes: copied as
 // they are and put in order on the device -- interleaving 6 MB on the host took
-// longer than the copy.  The kernel layout is kept where an adjoint needs it,
-// else only on the way to the spectral core's.  On the plan's device, whichever is
-// current.  Done on return.
+// longer than the copy.  Sets up to kPackElems are put together with their eigenvalues on
+// the host instead: a copy from pageable memory takes about 10 us whatever its size (two
+// planes of 2312, 6936 and 12696 values: 37, 42 and 46 us by three copies, 25, 34 and 47
+// put together).
+// The kernel layout is kept where an adjoint needs it, else only on the way to the
+// spectral core's.  On the plan's device, whichever is current.  Done on return.
+constexpr size_t kPackElems = 12288;
 int upload_kernels(kl_socs_plan p, int set, const float* re, const float* im, const float* scales) {
   const kl::OnDevice on(p->device);
   KL_CUDA_TRY(on.status);
   const size_t n = (size_t)p->g.nby * p->g.nbx * p->K, k0 = (size_t)set * p->K;
+  const bool pack = n <= kPackElems && !p->H;
   void* tmp = nullptr;
-  const size_t tmp_floats = (p->H ? 0 : 2 * n) + (im ? 2 * n : 0);
+  const size_t tmp_floats = pack ? 2 * n + p->K : (p->H ? 0 : 2 * n) + (im ? 2 * n : 0);
   int rc = tmp_floats ? kl::scratch_alloc(&tmp, sizeof(float) * tmp_floats, nullptr, "kernels") : KL_OK;
   if (rc) return rc;
   float2* H = p->H ? p->H + set * n : static_cast<float2*>(tmp);
   float* planes = static_cast<float*>(tmp) + (p->H ? 0 : 2 * n);
-  auto copy = [&](void* dst, const void* src, size_t bytes) {
-    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  auto copy = [&](void* dst, const void* src, size_t bytes, cudaMemcpyKind kind = cudaMemcpyHostToDevice) {
+    const cudaError_t e = kind == cudaMemcpyHostToDevice ? cudaMemcpy(dst, src, bytes, kind)
+                                                         : cudaMemcpyAsync(dst, src, bytes, kind, nullptr);
     if (e == cudaSuccess) return KL_OK;
     kl::set_error(std::string("kl_socs_set_kernels: ") + cudaGetErrorString(e));
     return KL_ERR_CUDA;
   };
-  if (im) {
+  if (pack) {
+    std::vector<float> h(tmp_floats);
+    if (im) {
+      for (size_t i = 0; i < n; ++i) {
+        h[2 * i] = re[i];
+        h[2 * i + 1] = im[i];
+      }
+    } else {
+      std::memcpy(h.data(), re, sizeof(float2) * n);
+    }
+    std::memcpy(h.data() + 2 * n, scales, sizeof(float) * p->K);
+    rc = copy(tmp, h.data(), sizeof(float) * tmp_floats);
+  } else if (im) {
     if (!(rc = copy(planes, re, sizeof(float) * n)) && !(rc = copy(planes + n, im, sizeof(float) * n)))
       rc = kl::spec_interleave(planes, planes + n, n, H, nullptr);
   } else {
     rc = copy(H, re, sizeof(float2) * n);
   }
   if (!rc) rc = kl::spec_columns(p->sg, H, p->K, p->HT + k0 * kl::spec_kernel_elems(p->sg), nullptr);
-  if (!rc) rc = copy(p->lam + k0, scales, sizeof(float) * p->K);
+  if (!rc)
+    rc = pack ? copy(p->lam + k0, H + n, sizeof(float) * p->K, cudaMemcpyDeviceToDevice)
+              : copy(p->lam + k0, scales, sizeof(float) * p->K);
   if (!rc && cudaStreamSynchronize(nullptr) != cudaSuccess) {
     kl::set_error(std::string("kl_socs_set_kernels: ") + cudaGetErrorString(cudaGetLastError()));
     rc = KL_ERR_CUDA;

@@ -17,6 +17,10 @@ extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = t_device; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { t_device = d; return cudaSuccess; }
 cudaError_t cudaMemcpy(void* a, const void* b, size_t n, cudaMemcpyKind) { std::memcpy(a, b, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void* a, const void* b, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(a, b, n);
+  return cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }

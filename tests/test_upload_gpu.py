@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("Lx,Ly,Nx,Ny,nk,nsets", [
-    (512, 512, 8, 8, 3, 2), (127, 40, 0, 2, 1, 1), (260, 300, 31, 7, 4, 2), (300, 310, 32, 37, 2, 2)])
+    (512, 512, 8, 8, 3, 2), (127, 40, 0, 2, 1, 1), (260, 300, 31, 7, 4, 2), (300, 310, 32, 37, 2, 2), (512, 520, 55, 55, 2, 1), (300, 310, 32, 37, 1, 1)])
 def test_planes_and_interleaved(cuda, Lx, Ly, Nx, Ny, nk, nsets):
     import torch
     plans = [K.SocsPlan(Lx, Ly, Nx, Ny, nk, nsets=nsets, max_clips=1, adjoint=True) for _ in range(2)]
