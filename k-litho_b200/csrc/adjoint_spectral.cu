@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(128, 2)
   const int img = blockIdx.x / CL, c0 = (blockIdx.x - img * CL) * RC, split = blockIdx.y;
   const int clip = img / nsets, set = img - clip * nsets;
   const int k0 = (int)(((long long)K * split) / nsplit), k1 = (int)(((long long)K * (split + 1)) / nsplit);
+  // last kernel first, as in k_spectral: the smallest weights are added up first
   const int nbatch = (k1 - k0 + KB - 1) / KB;
 
   // both halves: kernel slot, x residue, band row; each its own feed of the kernel
@@ -186,12 +187,12 @@ __global__ void __launch_bounds__(128, 2)
   if (rowthr) {
     hleft = (k1 - k0 - slot1 + KB - 1) / KB;
     if (hleft > 0) {
-      hk = H + ((size_t)set * K + k0 + slot1) * hs + row1;
+      hk = H + ((size_t)set * K + (k1 - 1 - slot1)) * hs + row1;
       h0 = __ldg(hk);
     }
     feed.h = hleft > 0 ? hk + spec_n0(g) + row1 : H;
     feed.pair = 2 * nby;
-    feed.skip = (ptrdiff_t)((KB - 1) * hs) + spec_n0(g);
+    feed.skip = spec_n0(g) - (ptrdiff_t)((KB + 1) * hs);
     feed.ring = (unsigned)__cvta_generic_to_shared(myring);
     feed.q = feed.put = 0;
     feed.left = hleft;
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(128, 2)
   };
   auto next_h0 = [&] {
     if (--hleft > 0) {
-      hk += (size_t)KB * hs;
+      hk -= (size_t)KB * hs;
       h0 = __ldg(hk);
     } else {
       h0 = make_float2(0.f, 0.f);
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(128, 2)
       }
     } else if (rowthr && b > 0) {  // back transform of batch b - 1
       const int k2 = (b - 1) * KB + slot1;
-      const float lk = k2 < k1 - k0 ? __ldg(lams + k2) * invg2 : 0.f;
+      const float lk = k2 < k1 - k0 ? __ldg(lams + (k1 - k0 - 1 - k2)) * invg2 : 0.f;
       float2 v[32];
       const float2* z = Z + ((size_t)(slot1 * RC + cc1) * RG * 32 + (row1 & 31)) * kP;
 #pragma unroll
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(128) k_adjoint_grad(const float2* gam, const S
     const float2* p1 = gam + (size_t)clip * nparts * nb2 + (size_t)(a + g.Ny) * g.nbx + (b + g.Nx);
     const float2* p2 = gam + (size_t)clip * nparts * nb2 + (size_t)(g.Ny - a) * g.nbx + (g.Nx - b);
 #pragma unroll 16
-    for (int p = 0; p < nparts; ++p) {
+    for (int p = nparts - 1; p >= 0; --p) {
       f1 = cadd(f1, p1[p * nb2]);
       f2 = cadd(f2, p2[p * nb2]);
     }
