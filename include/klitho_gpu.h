@@ -272,7 +272,9 @@ int kl_socs_stage_times(kl_socs_plan plan, double* ms, int* launches);
  * images (nclips x Ly x Lx float32), all device memory -- and the scratch
  * comes from one static 8 MiB device array inside the library (about 38 clips
  * of 1024^2 per call; larger requests return KL_ERR_INVALID with the sizes in
- * kl_last_error).  The first call on each device looks up that array's
+ * kl_last_error) and, for partial sums, from images_dev itself, which holds
+ * nothing of use until the call's work is done (it may be masks_dev, which is
+ * read before).  The first call on each device looks up that array's
  * device address; make it before any stream capture.  The address is looked
  * up again when the device's primary context has changed since (after a
  * cudaDeviceReset); make the first call after such a reset outside a capture

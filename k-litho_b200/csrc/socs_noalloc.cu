@@ -7,7 +7,8 @@
 // kl_socs_forward_noalloc serves them: the caller owns every input and output
 // buffer, and the pipeline's scratch (strip partial spectra, intensity
 // spectra, twiddle tables) lives in one fixed-size file-scope device array
-// below instead of in cudaMalloc'd plan buffers.
+// below instead of in cudaMalloc'd plan buffers, and the spectral core's partial
+// sums pass through the image buffer before the images are written to it.
 //
 // The array is part of the module: every GPU that loads the library holds it
 // (kNoallocScratchBytes) until the process exits.  All calls share it and it
@@ -102,7 +103,8 @@ extern "C" int kl_socs_forward_noalloc(const float* masks_dev, int nclips, int L
   const size_t b_tx = up256(sizeof(float2) * kl::socs_table_x_elems(g));
   const size_t b_ty = up256(sizeof(float2) * kl::socs_table_y_elems(g));
   const size_t b_part = up256(kl::socs_partial_bytes(g, nclips));
-  // a call's budget counts the spectra of the kernel slices (up to 8) of few clips
+  // a call's budget counts the spectra of up to 8 kernel slices of few clips, as it did
+  // when they were kept here: what is refused does not depend on where they pass
   int slices = 1;
   while (slices < 8 && nclips * slices < 2 * 148 && nk / (2 * slices) >= 3) slices *= 2;
   const size_t b_T = up256(sizeof(float2) * (size_t)nclips * slices * g.nty * g.ntx);

@@ -83,3 +83,23 @@ def test_noalloc_rejects_oversized_request(cuda):
            dummy.data_ptr(), None)
     assert rc == K.KL_ERR_INVALID
     assert "static workspace" in K.last_error()
+
+
+@pytest.mark.parametrize("L,n,nk,shift", [(512, 3, 24, 0), (1024, 1, 24, 0), (512, 2, 7, 4), (1024, 2, 64, 60)])
+def test_noalloc_images_over_masks(cuda, L, n, nk, shift):
+    """The image buffer, which the call also uses for partial sums, may be the masks'; it
+    may start at any float."""
+    import torch
+    f = _noalloc()
+    c = _case(L, n, nk, seed=3)
+    room = torch.zeros(n * L * L + 64, dtype=torch.float32, device="cuda")
+    at = shift // 4
+    c["out"] = room[at:at + n * L * L].view(n, L, L)
+    c["out"].copy_(c["md"])
+    if shift == 0:
+        c["md"] = c["out"]
+    _call(f, c)
+    torch.cuda.synchronize()
+    assert np.abs(c["out"].cpu().numpy() - c["ref"].cpu().numpy()[:, 0]).max() <= TOL_CF * c["cf"]
+    assert float(room[:at].abs().sum()) == 0 and float(room[at + n * L * L:].abs().sum()) == 0
+    c["plan"].close()
