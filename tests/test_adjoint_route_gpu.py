@@ -40,3 +40,27 @@ def test_adjoint_both_sides(cuda, clips, nsets, mode):
             assert np.abs(img[c, s].cpu().numpy() - I).max() <= 1e-5 * np.abs(I).max()
         assert np.abs(grad[c].cpu().numpy() - gr).max() <= 1e-4 * np.abs(gr).max()
         assert abs(float(loss.reshape(clips, nsets)[c].sum()) - nsets * lo) <= 1e-4 * nsets * lo
+
+
+@pytest.mark.parametrize("clips,nsets,few", [(16, 1, True), (17, 1, False), (8, 2, True), (9, 2, False)])
+def test_auto_takes_the_engine_of_its_size(cuda, clips, nsets, few):
+    """Up to 64 tiles the automatic choice gives the CUDA cores' images bit for bit, above
+    them others (the tensor cores'; tensor mode has another mask transform too)."""
+    import torch
+    L, N, k = 512, 6, 3
+    krn, sc = synth.random_kernels(k, N, N, seed=5)
+    md = torch.from_numpy(np.stack([synth.smooth_mask(L, seed=s, sigma_px=3.0) for s in range(clips)])).cuda()
+    td = (md > 0.5).float()
+    images = {}
+    plan = K.SocsPlan(L, L, N, N, k, nsets=nsets, max_clips=clips, adjoint=True)
+    for s in range(nsets):
+        plan.set_kernels(s, krn, sc)
+    for mode in ("auto", "cuda", "tensor"):
+        plan.set_synthesis(mode)
+        images[mode] = torch.zeros((clips, nsets, L, L), dtype=torch.float32, device="cuda")
+        plan.vjp(md, td, torch.empty_like(md), torch.empty(clips * nsets, dtype=torch.float64, device="cuda"), images[mode])
+        torch.cuda.synchronize()
+    plan.status()
+    plan.close()
+    assert not torch.equal(images["cuda"], images["tensor"])
+    assert torch.equal(images["auto"], images["cuda"]) == few
