@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256) k_chol_inv(const double2* __restrict__ G,
 // holds entries (ty + 16 a, tx + 16 b).  Latency of one CTA: a step is one barrier, a
 // row exchanged through shared memory, and NB^2 independent updates; rows stay
 // unscaled (L D L^H) until the end.  36 columns took 81 us in the kernel above, and 57
-// us at 48 with its updates on shared memory; here 11.
+// us at 48 with its updates on shared memory; here 26 us at 48 columns.
 template <int NB>
 __global__ void __launch_bounds__(256) k_chol_inv_reg(const double2* __restrict__ G, int B, double rel_shift,
                                                       double2* __restrict__ Rinv, int* __restrict__ status) {

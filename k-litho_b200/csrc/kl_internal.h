@@ -154,7 +154,11 @@ __host__ __device__ inline bool gen_t2_in_smem(const GenGeom& g) { return (size_
 // (P = 1), 2002, 2004 and 1992 pixels, four clips of 1203 rows, 55 (synthesis of 8
 // images) and 28 bins (mask transform), us: synthesis 444, 212, 115, 63 by FFTs, 94 by
 // products; mask transform 150, 81, 55, 32 against 79; image, resist and transform of
-// dL/dI 601, 314, 170, 99 against 215.
+// dL/dI 601, 314, 170, 99 against 215.  Whole calls at about 500, 1000 and 2000 pixels, 3 to
+// 55 frequencies, 1 and 8 clips, the other side's time over this side's: synthesis at
+// P = 4 0.99 to 1.23, at P = 8 1.02 to 1.39; transforms at P = 2 with 8 clips 1.05 to 1.50
+// (with one, which leaves most SMs without a tile, 0.80 to 1.12), at P = 4 with one clip
+// 1.11 to 1.74 (with 8, 0.82 to 1.11).
 inline bool gen_direct_synth(const GenGeom& g) { return g.P <= 4 && g.ntx <= 112; }
 inline bool gen_direct_dft(const GenGeom& g) { return g.P <= 2 && g.ntx <= 112; }
 const float2* gen_roots_x(const GenGeom& g, const float2* tables);  // e^{+2 pi i m / Lx}

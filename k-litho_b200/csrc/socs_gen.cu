@@ -28,8 +28,6 @@
 // Twiddle tables that depend on the period are made once per plan with exact
 // double-precision arguments.  Only row bins (Nx+1 or 2Nx+1 per row), band
 // partials and T pass through global memory.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <climits>
 
@@ -38,8 +36,6 @@
 #include "kl_internal.h"
 #include "kl_launch.cuh"
 #include "row_fold.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace kl {
 

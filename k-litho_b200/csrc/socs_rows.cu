@@ -4,7 +4,7 @@
 // A row has a few dozen bins and a thousand pixels, and the register FFTs of
 // socs_gen.cu shrink with the power of two in Lx: at odd widths every pixel meets
 // every bin, with a twiddle and a coefficient from shared memory each time (1.16 ms for
-// 24 images of 2001 x 1203, 16 us of HBM traffic per image).  These kernels are the
+// 24 images of 2001 x 1203, 1.5 us of HBM traffic each).  These kernels are the
 // same sums as register-tiled matrix products:
 //   * pixels x and Lx - x share a product (cos even, sin odd in x):
 //     sum_b Re(q_b w^{bx}) = C -+ S, C = sum a_b cos, S = sum b_b sin;
