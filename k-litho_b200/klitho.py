@@ -316,7 +316,8 @@ class SocsPlan:
 
     def autotune(self, masks_dev, images_dev, nclips: int | None = None, stream=None):
         """Pick the fastest launch shape for batches of nclips clips
-        (kl_socs_autotune); returns (kernel slices, strips per CTA)."""
+        (kl_socs_autotune); returns (the fastest of 1, 2, 4 and 8 kernel slices,
+        strips per CTA), also where the plan keeps its untuned slice count."""
         n = masks_dev.shape[0] if nclips is None else nclips
         ns, spc = ctypes.c_int(), ctypes.c_int()
         check(lib().kl_socs_autotune(self._h, _dev_ptr(masks_dev), int(n), _dev_ptr(images_dev),
